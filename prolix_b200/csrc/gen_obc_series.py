@@ -14,12 +14,21 @@ that minimises the largest RELATIVE error on [0, u_max] (Remez exchange),
 which needs far fewer terms for the same bound: 6 terms reach 2e-8 up to
 u = 0.16 where the Taylor series needs 10.
 
-Run:  python prolix_b200/csrc/gen_obc_series.py   (rewrites the header)
+The FP64 energy path evaluates V in the same tiers, and 2^-g on
+[-1/2, 1/2], in double precision: there each polynomial interpolates at the
+Chebyshev nodes of its interval (within a few units of the minimax error at
+these degrees), solved in rational arithmetic so that the coefficients carry
+no rounding but their own (pb2_series64.cuh).
+
+Run:  python prolix_b200/csrc/gen_obc_series.py   (rewrites both headers)
 """
 
 from __future__ import annotations
 
+import decimal
+import math
 import os
+from fractions import Fraction
 
 import numpy as np
 
@@ -30,6 +39,10 @@ import numpy as np
 VALUE_TIERS = ((3, 0.0075), (4, 0.036), (5, 0.089), (6, 0.16))
 DERIV_TIERS = ((4, 0.027), (5, 0.07), (6, 0.129), (7, 0.16))
 REL_BOUND = 2e-8
+# FP64: terms of V on each value tier and of 2^-g; the bound is 1.5 ulp
+VALUE_TERMS64 = (6, 8, 10, 12)
+EXP2_TERMS64 = 11
+REL_BOUND64 = 3.2e-16
 
 
 def exact(u, der: bool, n_terms: int = 300) -> np.ndarray:
@@ -110,8 +123,86 @@ def header() -> str:
   return "\n".join(out) + "\n"
 
 
+def _value_exact(u: Fraction) -> Fraction:
+  """V(u) to 1e-30 (u <= 0.16)."""
+  return sum(Fraction(k, 2 * k + 1) * u ** (k - 1) for k in range(1, 42))
+
+
+def _exp2neg_exact(g: Fraction) -> Fraction:
+  with decimal.localcontext() as c:
+    c.prec = 50
+    x = decimal.Decimal(g.numerator) / decimal.Decimal(g.denominator)
+    return Fraction((-x * decimal.Decimal(2).ln()).exp())
+
+
+def interpolant(f, lo: float, hi: float, n_terms: int):
+  """Coefficients (ascending powers, as FP64) of the polynomial through f at
+  the n_terms Chebyshev nodes of [lo, hi], and the largest relative error of
+  the exact polynomial with the rounded coefficients on a grid."""
+  nodes = [Fraction(0.5 * (lo + hi) + 0.5 * (hi - lo) * math.cos(math.pi * (2 * k + 1) / (2 * n_terms)))
+           for k in range(n_terms)]
+  d = [f(x) for x in nodes]  # divided differences
+  for j in range(1, n_terms):
+    for k in range(n_terms - 1, j - 1, -1):
+      d[k] = (d[k] - d[k - 1]) / (nodes[k] - nodes[k - j])
+  c = [Fraction(0)] * n_terms  # Newton form to powers
+  for k in range(n_terms - 1, -1, -1):
+    c = [d[k] - nodes[k] * c[0]] + [c[j - 1] - nodes[k] * c[j] for j in range(1, n_terms)]
+  c = [float(v) for v in c]
+  worst = 0.0
+  for t in range(201):
+    x = Fraction(lo + (hi - lo) * t / 200)
+    p = Fraction(0)
+    for v in reversed(c):
+      p = p * x + Fraction(v)
+    y = f(x)
+    worst = max(worst, abs(float((p - y) / y)))
+  return c, worst
+
+
+def header64() -> str:
+  out = [
+      "// Generated by gen_obc_series.py; do not edit.",
+      "//",
+      "// FP64 polynomials of the energy path: the OBC far-field series V(u) on the",
+      "// value tiers of pb2_obc_series.cuh, and 2^-g on [-1/2, 1/2].  In exact",
+      f"// arithmetic each is within {REL_BOUND64:.1e} relative of its function.",
+      "#pragma once",
+      "",
+      "namespace pb2 {",
+      "",
+      "template <int TIER>",
+      "struct ObcPoly64;",
+      "",
+  ]
+
+  def body(arg, coef):
+    out.append(f"  double p = {coef[-1]!r};")
+    for c in reversed(coef[:-1]):
+      out.append(f"  p = fma(p, {arg}, {c!r});")
+    out.append("  return p;")
+
+  for tier, ((_, u_max), n) in enumerate(zip(VALUE_TIERS, VALUE_TERMS64)):
+    coef, err = interpolant(_value_exact, 0.0, u_max, n)
+    if err > REL_BOUND64:
+      raise SystemExit(f"FP64 tier {tier}: {err:.3e} > {REL_BOUND64}")
+    out.append(f"// V(u), u <= {u_max}: {n} terms, relative error {err:.1e}")
+    out += ["template <>", f"struct ObcPoly64<{tier}> {{", "  __device__ __forceinline__ static double eval(double u) {"]
+    body("u", coef)
+    out += ["  }", "};", ""]
+  coef, err = interpolant(_exp2neg_exact, -0.5, 0.5, EXP2_TERMS64)
+  if err > REL_BOUND64:
+    raise SystemExit(f"FP64 2^-g: {err:.3e} > {REL_BOUND64}")
+  out.append(f"// 2^-g, |g| <= 1/2: {EXP2_TERMS64} terms, relative error {err:.1e}")
+  out.append("__device__ __forceinline__ double exp2neg_poly(double g) {")
+  body("g", coef)
+  out += ["}", "", "}  // namespace pb2"]
+  return "\n".join(out) + "\n"
+
+
 if __name__ == "__main__":
-  path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "pb2_obc_series.cuh")
-  with open(path, "w") as f:
-    f.write(header())
-  print("wrote", path)
+  for name, text in (("pb2_obc_series.cuh", header), ("pb2_series64.cuh", header64)):
+    path = os.path.join(os.path.dirname(os.path.abspath(__file__)), name)
+    with open(path, "w") as f:
+      f.write(text())
+    print("wrote", path)

@@ -223,19 +223,6 @@ static void spatial_order(const double *pos, int n, std::vector<int> &ord) {
   for (int a = 0; a < n; a += 32) std::sort(ord.begin() + a, ord.begin() + std::min(n, a + 32));
 }
 
-static std::vector<TileItem> build_items(const std::vector<SysInfo> &sinfo, int seg) {
-  std::vector<TileItem> items;
-  for (int s = 0; s < (int)sinfo.size(); ++s) {
-    const int nblk = sinfo[s].nblk;
-    for (int ib = 0; ib < nblk; ++ib)
-      for (int j0 = ib; j0 < nblk; j0 += seg) items.push_back(TileItem{s, ib, j0, std::min(j0 + seg, nblk)});
-  }
-  std::stable_sort(items.begin(), items.end(), [](const TileItem &p, const TileItem &q) {
-    return (p.jb1 - p.jb0) > (q.jb1 - q.jb0);
-  });
-  return items;
-}
-
 // Work items of the two-i-block force kernel: even i-blocks ib (with ib + 1)
 // against j-blocks [j0, j1), j0 >= ib.
 static std::vector<TileItem> build_items2(const std::vector<SysInfo> &sinfo, int seg) {
@@ -248,6 +235,32 @@ static std::vector<TileItem> build_items2(const std::vector<SysInfo> &sinfo, int
   std::stable_sort(items.begin(), items.end(), [](const TileItem &p, const TileItem &q) {
     return (p.jb1 - p.jb0) > (q.jb1 - q.jb0);
   });
+  return items;
+}
+
+// Items of the FP64 energy kernels: pairs of i-blocks.  Each item's sums are
+// rounded to fixed point once, so how a system is cut depends on its own size
+// alone and its energies are the same in every batch.  A small system has
+// its tiles' 32 steps shared by 8, 4 or 2 items (as many as one resident
+// wave of 1,776 warps holds): what it waits for is its longest item.  A large
+// one takes several tiles per item, which load their i atoms once.
+static std::vector<TileItem> build_items_e64(const std::vector<SysInfo> &sinfo) {
+  std::vector<TileItem> items;
+  for (int s = 0; s < (int)sinfo.size(); ++s) {
+    const int nblk = sinfo[s].nblk;
+    const int parts = nblk <= 28 ? 8 : nblk <= 40 ? 4 : nblk <= 57 ? 2 : 1;  // 224, 440, 870 tiles
+    const int seg = nblk < 160 ? 1 : nblk < 256 ? 2 : nblk < 400 ? 4 : 8;
+    const int kn = 32 / parts;
+    for (int ib = 0; ib < nblk; ib += 2)
+      for (int j0 = ib; j0 < nblk; j0 += seg)
+        for (int p = 0; p < parts; ++p)
+          items.push_back(TileItem{s, ib, j0, parts > 1 ? part_code(p * kn, kn) : std::min(j0 + seg, nblk)});
+  }
+  auto cost = [](const TileItem &t) {
+    const ItemRange r = item_range(t);
+    return (r.jb1 - r.jb0) * r.kn;
+  };
+  std::stable_sort(items.begin(), items.end(), [&](const TileItem &p, const TileItem &q) { return cost(p) > cost(q); });
   return items;
 }
 
@@ -679,8 +692,12 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
     hkeys[2 * (size_t)s + 1] = d.key[1];
     blk_base += S.nblk;
   }
-  hitems = build_items(sinfo, b->params.tile_segment);
-  b->n_items = (int)hitems.size();
+  {
+    hitems = build_items_e64(sinfo);
+    b->n_items = (int)hitems.size();
+    for (int p = 0; p < 2; ++p)
+      b->grid_e64[p] = std::max(1, std::min(energy64_occupancy(p) * ctx->sm_count, b->n_items));
+  }
   b->sys_host = sinfo;
 
   // --- bonded tables (global atom indices)
@@ -790,7 +807,7 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   b->par = D.alloc<float4>(N);
   b->born = D.alloc<float4>(N);
   b->bbox = D.alloc<float4>(2 * (size_t)blocks_total);
-  b->sched = D.alloc<int32_t>(8);
+  b->sched = D.alloc<int32_t>(kSchedWords);
   b->blk_sys = D.alloc<int32_t>(blocks_total);
   b->blk_info = D.alloc<int4>(blocks_total);
   b->n_blocks = blocks_total;
@@ -822,6 +839,7 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   b->user = D.alloc<int32_t>(N);
   b->devidx = D.alloc<int32_t>(N);
   b->born_acc = D.alloc<long long>(N);
+  b->born_acc64 = D.alloc<long long>(N);
   b->dedb_acc = D.alloc<long long>(N);
   b->energy = D.alloc<long long>((size_t)n_systems * PB2_NTERMS);
   b->keys = D.alloc<uint32_t>(4 * (size_t)n_systems);
@@ -887,10 +905,11 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   CUDA_TRY(ctx, cudaMemset(b->fy, 0, N * sizeof(long long)));
   CUDA_TRY(ctx, cudaMemset(b->fz, 0, N * sizeof(long long)));
   CUDA_TRY(ctx, cudaMemset(b->born_acc, 0, N * sizeof(long long)));
+  CUDA_TRY(ctx, cudaMemset(b->born_acc64, 0, N * sizeof(long long)));
   CUDA_TRY(ctx, cudaMemset(b->dedb_acc, 0, N * sizeof(long long)));
   CUDA_TRY(ctx, cudaMemset(b->born, 0, N * sizeof(float4)));
   CUDA_TRY(ctx, cudaMemset(b->steps, 0, n_systems * sizeof(long long)));
-  CUDA_TRY(ctx, cudaMemset(b->sched, 0, 8 * sizeof(int32_t)));
+  CUDA_TRY(ctx, cudaMemset(b->sched, 0, kSchedWords * sizeof(int32_t)));
   CUDA_TRY(ctx, cudaMemset(b->status, 0, n_systems * sizeof(uint32_t)));
   CUDA_TRY(ctx, cudaMemset(b->guard_end, 0, sizeof(int32_t)));
   CUDA_TRY(ctx, cudaMemset(b->warn_flags, 0, 2 * (size_t)n_systems * sizeof(uint32_t)));
@@ -986,10 +1005,7 @@ static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_ene
     fa.born_acc = b->born_acc;
     fa.born = b->born;
     fa.dedb_acc = b->dedb_acc;
-    fa.energy = b->energy;
-    fa.born64 = nullptr;
     fa.n_total = b->n_total;
-    fa.energy_mode = 0;
     fa.blk_sys = b->blk_sys;
     fa.n_blocks = b->n_blocks;
     fa.sys_fin = b->sys_fin;
@@ -1052,28 +1068,20 @@ static cudaError_t enqueue_energy64(pb2_batch *b, cudaStream_t st) {
   ea.excl_rows = b->excl_rows;
   ea.x = b->x; ea.y = b->y; ea.z = b->z;
   ea.q = b->q64; ea.hs = b->hs64; ea.se = b->se64; ea.ro = b->ro64; ea.sr = b->sr64;
+  ea.radius = b->radius;
   ea.born64 = b->born64;
-  ea.born_acc = b->born_acc;
+  ea.born_acc = b->born_acc64;
   ea.energy = b->energy;
-  const int grid = b->grid_pair[PASS_FORCE];
+  ea.bbox = b->bbox;
+  ea.blk_sys = b->blk_sys;
+  ea.n_blocks = b->n_blocks;
+  ea.sched = b->sched + kSchedE64;
   if (b->params.terms & PB2_USE_GB) {
-    if ((e = cudaMemsetAsync(b->born_acc, 0, (size_t)b->n_total * sizeof(long long), st)) != cudaSuccess) return e;
-    if ((e = launch_energy64(0, ea, grid, st)) != cudaSuccess) return e;
-    FinalizeArgs fa;
-    fa.sys = b->sys;
-    fa.atom_sys = b->atom_sys;
-    fa.radius = b->radius;
-    fa.charge = b->charge;
-    fa.born_acc = b->born_acc;
-    fa.born = b->born;
-    fa.dedb_acc = b->dedb_acc;
-    fa.energy = b->energy;
-    fa.born64 = b->born64;
-    fa.n_total = b->n_total;
-    fa.energy_mode = 1;
-    if ((e = launch_born_finalize(fa, st)) != cudaSuccess) return e;
+    if ((e = launch_energy64(0, ea, b->grid_e64[0], st)) != cudaSuccess) return e;
+    if ((e = launch_finalize64(ea, st)) != cudaSuccess) return e;
   }
-  return launch_energy64(1, ea, grid, st);
+  ea.sched = b->sched + kSchedE64 + 2;
+  return launch_energy64(1, ea, b->grid_e64[1], st);
 }
 
 static int fresh_forces(pb2_batch *b, cudaStream_t st, bool energy) {
@@ -1879,13 +1887,7 @@ extern "C" int pb2_set_tile_segment(pb2_batch *b, int32_t segment) {
   pb2_ctx *ctx = b->ctx;
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   if (segment == b->params.tile_segment) return PB2_OK;
-  std::vector<TileItem> items = build_items(b->sys_host, segment);
   CUDA_TRY(ctx, cudaDeviceSynchronize());
-  b->dev.release(b->items);
-  b->items = b->dev.alloc<TileItem>(items.size());
-  if (!b->items) return fail(ctx, PB2_ENOMEM, "work-item allocation failed");
-  CUDA_TRY(ctx, cudaMemcpy(b->items, items.data(), items.size() * sizeof(TileItem), cudaMemcpyHostToDevice));
-  b->n_items = (int)items.size();
   b->params.tile_segment = segment;
   if (int rc = setup_items2(b, segment)) return rc;
   if (int rc = setup_pair_list(b, segment)) return rc;

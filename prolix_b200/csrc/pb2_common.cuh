@@ -62,10 +62,21 @@ struct SysInfo {
 static_assert(sizeof(SysInfo) == 168, "SysInfo layout");
 
 // Work item of the tile kernels: tiles (iblk, jb) for jb in [jb0, jb1) of
-// system sys.  Block indices are local to the system.
+// system sys.  Block indices are local to the system.  A tile's 32 steps can
+// be shared between items: jb1 = part_code(k0, kn) < 0 stands for steps
+// k0 .. k0 + kn - 1 of the one tile (iblk, jb0).
 struct TileItem {
   int32_t sys, iblk, jb0, jb1;
 };
+struct ItemRange {
+  int jb0, jb1, k0, kn;
+};
+__host__ __device__ __forceinline__ int32_t part_code(int k0, int kn) { return ~(k0 | (kn << 5)); }
+__host__ __device__ __forceinline__ ItemRange item_range(const TileItem &t) {
+  if (t.jb1 >= 0) return ItemRange{t.jb0, t.jb1, 0, 32};
+  const int c = ~t.jb1;
+  return ItemRange{t.jb0, t.jb0 + 1, c & 31, c >> 5};
+}
 
 // One row of the pair list: the even i-block iblk (with iblk + 1) of system
 // sys; its live j-blocks are stored from pair_list_j[jbase], room for

@@ -72,7 +72,7 @@ struct pb2_batch {
   double *mass = nullptr, *sigma = nullptr, *charge = nullptr, *radius = nullptr;
   float4 *posq = nullptr, *par = nullptr, *born = nullptr, *bbox = nullptr;
   int32_t *blk_sys = nullptr;
-  int32_t *sched = nullptr;  // per pass: (next item, finished warps)
+  int32_t *sched = nullptr;  // per pass (pair passes, then the FP64 energy passes): (next item, finished warps)
   int n_blocks = 0;
   double *q64 = nullptr, *hs64 = nullptr, *se64 = nullptr, *ro64 = nullptr, *sr64 = nullptr;
   double *born64 = nullptr;
@@ -99,8 +99,10 @@ struct pb2_batch {
   int32_t *guard_end = nullptr;
   uint32_t *warn_flags = nullptr;
   int32_t *warn_counts = nullptr;
-  TileItem *items = nullptr;   // (i-block, j-range) items of the FP64 energy kernels
+  TileItem *items = nullptr;   // items of the FP64 energy kernels, every system's
   int n_items = 0;
+  int grid_e64[2] = {1, 1};    // their two passes' grids
+  long long *born_acc64 = nullptr;  // their descreening sums
   TileItem *items2 = nullptr;  // pair kernels: the live items (those of systems not retired)
   TileItem *items2_all = nullptr;  // every system's items over pairs of i-blocks
   int n_items2 = 0;                // items in items2_all

@@ -39,6 +39,8 @@ struct BondedArgs {
   const double4 *exc_par;  // (k_coulomb * charge product, sigma, epsilon, 0)
 };
 enum { PASS_BORN = 0, PASS_FORCE = 1, PASS_CHAIN = 2 };
+// batch sched words: two per pair pass, then two per FP64 energy pass
+constexpr int kSchedE64 = 6, kSchedWords = 12;
 struct FinalizeArgs {
   const SysInfo *sys;
   const int32_t *atom_sys;
@@ -47,10 +49,7 @@ struct FinalizeArgs {
   long long *born_acc;
   float4 *born;
   long long *dedb_acc;
-  long long *energy;
-  double *born64;   // NULL, or FP64 Born radii out
   int32_t n_total;
-  int32_t energy_mode;
   // finalize as the descreening pass's tail chunks (one per 32-atom block)
   const int32_t *blk_sys;
   int32_t n_blocks;
@@ -124,9 +123,14 @@ struct Energy64Args {
   const ExclRow *excl_rows;
   const double *x, *y, *z;
   const double *q, *hs, *se, *ro, *sr;  // charge, sigma/2, sqrt(eps), rho~, scaled radius
-  const double *born64;
-  long long *born_acc;
+  const double *radius;
+  double *born64;
+  long long *born_acc;   // this path's own descreening sums; zero between evaluations
   long long *energy;
+  const float4 *bbox;
+  const int32_t *blk_sys;
+  int32_t n_blocks;
+  int32_t *sched;        // (items taken, finished warps); zero between launches
 };
 
 // Neighbour-list control words (NlArgs::ctl)
@@ -240,7 +244,11 @@ cudaError_t launch_lbfgs(int op, const LbfgsArgs &a, int last_trial, cudaStream_
 constexpr int kShapesPerPass = 3;
 int tile_shape(int pass, int shape, int *threads, int *min_blocks);
 cudaError_t launch_tiles(int pass, const PairArgs &a, int grid, int shape, cudaStream_t st);
+// The descreening (pass 0) and energy (pass 1) kernels, and between them the
+// FP64 Born radii with the per-atom energies.
 cudaError_t launch_energy64(int pass, const Energy64Args &a, int grid, cudaStream_t st);
+cudaError_t launch_finalize64(const Energy64Args &a, cudaStream_t st);
+int energy64_occupancy(int pass);
 cudaError_t launch_born_finalize(const FinalizeArgs &a, cudaStream_t st);
 int tile_kernel_occupancy(int pass, bool cut, int shape);
 int tile_kernel_warps(int pass, int shape);  // warps per block of a pair pass

@@ -571,41 +571,16 @@ __device__ __forceinline__ void run_bc_tile2(const PData2 &I, const JTile &jt, A
 
 // One atom's Born radius from its descreening sum, and the per-atom GB
 // self term and ACE as the initial dE/dB; clears the sum.
-__device__ __forceinline__ void finalize_atom(const FinalizeArgs &a, int i, int s, const SysInfo &S) {
-  const bool nl = S.clamp != 0;
+__device__ __forceinline__ void finalize_atom(const FinalizeArgs &a, int i, const SysInfo &S) {
   const double isum = (double)__ldcg(&a.born_acc[i]) * kBornInv;
   a.born_acc[i] = 0;
   const double r_in = a.radius[i];
-  const double rad = nl ? fmax(r_in, 1e-6) : r_in;
-  double ro = rad - kDielOffset;
-  if (nl) ro = fmax(ro, 1e-4);
-  const double psi = ro * isum;
-  const double arg = kObcAlpha * psi - kObcBeta * psi * psi + kObcGamma * psi * psi * psi;
-  const double th = tanh(arg);
-  const double dr = nl ? fmax(rad, 1e-4) : rad;
-  double inv_b = 1.0 / ro - th / dr;
-  bool clamped = false;
-  if (nl && inv_b < 1e-4) {
-    inv_b = 1e-4;
-    clamped = true;
-  }
-  const double B = 1.0 / inv_b;
-  const double dpsi = (kObcAlpha - 2.0 * kObcBeta * psi + 3.0 * kObcGamma * psi * psi) * ro;
-  const double dbdi = clamped ? 0.0 : B * B * (1.0 - th * th) / dr * dpsi;
-  a.born[i] = make_float4((float)B, (float)inv_b, (float)dbdi, 0.f);
-  if (a.born64) a.born64[i] = B;
+  const BornRadius R = born_radius(isum, r_in, S.clamp != 0);
+  a.born[i] = make_float4((float)R.B, (float)R.inv_b, (float)R.dbdi, 0.f);
   const double q = a.charge[i];
-  const double r_nm = (r_in - kDielOffset) / 10.0 + 0.009;
-  const double x = r_nm / (B / 10.0);
-  const double x3 = x * x * x;
-  const double ace = kAceCoeff * (r_nm + 0.14) * (r_nm + 0.14) * x3 * x3 * kKjToKcal;
-  const double dedb = -S.pref_d * q * q * inv_b * inv_b - 6.0 * ace * inv_b;
+  const double ace = ace_energy(r_in, R.B);
+  const double dedb = -S.pref_d * q * q * R.inv_b * R.inv_b - 6.0 * ace * R.inv_b;
   a.dedb_acc[i] = to_fix(dedb, kForceScale);
-  if (a.energy_mode) {
-    long long *e = a.energy + (size_t)s * PB2_NTERMS;
-    atomic_add_fix(&e[PB2_TERM_GB], to_fix(S.pref_d * q * q * inv_b, kEnergyScale));
-    atomic_add_fix(&e[PB2_TERM_NONPOLAR], to_fix(ace, kEnergyScale));
-  }
 }
 
 // Spins of the bounded waits (each a 128 ns sleep and an L2 read): about a
@@ -638,7 +613,7 @@ __device__ __noinline__ void finalize_chunk(const PairArgs &a, int c, const int3
   __threadfence();  // acquire: the counted items' sums are visible to every lane
   const int l = (c - S.blk_base) * 32 + lane;
   if (l < S.n) {
-    if (ok) finalize_atom(a.fin, S.off + l, s, S);
+    if (ok) finalize_atom(a.fin, S.off + l, S);
     else a.fin.born_acc[S.off + l] = 0;  // the next evaluation starts from zero all the same
   }
   __syncwarp();
@@ -654,8 +629,7 @@ __device__ __noinline__ void finalize_chunk(const PairArgs &a, int c, const int3
 
 __global__ void born_finalize(const FinalizeArgs a) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
-    const int s = a.atom_sys[i];
-    finalize_atom(a, i, s, a.sys[s]);
+    finalize_atom(a, i, a.sys[a.atom_sys[i]]);
   }
 }
 

@@ -43,6 +43,38 @@ __device__ __forceinline__ float obc_series_der_n(float u) {
   return p;
 }
 
+// An atom's Born radius from its descreening sum (generalized_born.py:61-94,
+// with the neighbour-list clamps of :300-337 when nl), in FP64.
+struct BornRadius {
+  double B, inv_b, dbdi;
+};
+__device__ __forceinline__ BornRadius born_radius(double isum, double r_in, bool nl) {
+  const double rad = nl ? fmax(r_in, 1e-6) : r_in;
+  double ro = rad - kDielOffset;
+  if (nl) ro = fmax(ro, 1e-4);
+  const double psi = ro * isum;
+  const double arg = kObcAlpha * psi - kObcBeta * psi * psi + kObcGamma * psi * psi * psi;
+  const double th = tanh(arg);
+  const double dr = nl ? fmax(rad, 1e-4) : rad;
+  double inv_b = 1.0 / ro - th / dr;
+  bool clamped = false;
+  if (nl && inv_b < 1e-4) {
+    inv_b = 1e-4;
+    clamped = true;
+  }
+  const double B = 1.0 / inv_b;
+  const double dpsi = (kObcAlpha - 2.0 * kObcBeta * psi + 3.0 * kObcGamma * psi * psi) * ro;
+  return BornRadius{B, inv_b, clamped ? 0.0 : B * B * (1.0 - th * th) / dr * dpsi};
+}
+
+// An atom's ACE energy (generalized_born.py:600-648).
+__device__ __forceinline__ double ace_energy(double r_in, double B) {
+  const double r_nm = (r_in - kDielOffset) / 10.0 + 0.009;
+  const double x = r_nm / (B / 10.0);
+  const double x3 = x * x * x;
+  return kAceCoeff * (r_nm + 0.14) * (r_nm + 0.14) * x3 * x3 * kKjToKcal;
+}
+
 // I(r; rho, s).  inv_r = 1/r (already available to every caller).
 __device__ __forceinline__ float obc_integral(float r, float inv_r, float rho, float s) {
   if (!(r + s > rho)) return 0.0f;
