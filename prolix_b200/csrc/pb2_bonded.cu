@@ -21,9 +21,26 @@
 
 namespace pb2 {
 
+// With energies wanted, a warp whose terms share one accumulator (nearly
+// every warp: terms are ordered by kind and atom) adds their fixed-point sum
+// once: the terms of a kind all meet at one address, and 80,000 atomics on
+// four addresses took 38 of the kernel's 43 us at N = 20,000.
 __global__ void bonded_kernel(const BondedArgs a) {
   const int total = bonded_total(a);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) bonded_term(a, t);
+  const int lane = threadIdx.x & 31;
+  for (int t0 = blockIdx.x * blockDim.x + threadIdx.x - lane; t0 < total; t0 += gridDim.x * blockDim.x) {
+    TermEnergy v{-1, 0};
+    if (t0 + lane < total) v = bonded_term(a, t0 + lane);
+    if (a.energy_mode) {  // uniform
+      int same = 0;
+      __match_all_sync(kFull, v.key, &same);
+      if (same) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v.e += __shfl_xor_sync(kFull, v.e, o);
+      }
+      if (v.key >= 0 && (!same || lane == 0)) atomic_add_fix(&a.energy[v.key], v.e);
+    }
+  }
 }
 
 cudaError_t launch_bonded(const BondedArgs &a, int grid_cap, cudaStream_t st) {

@@ -28,10 +28,15 @@ __device__ __forceinline__ void add_force(const BondedArgs &a, int i, D3 f) {
   atomic_add_fix(&a.fz[i], to_fix(f.z, kForceScale));
 }
 
-__device__ __forceinline__ void add_energy(const BondedArgs &a, int atom, int term, double e) {
-  if (!a.energy_mode) return;
-  const int s = a.atom_sys[atom];
-  atomic_add_fix(&a.energy[(size_t)s * PB2_NTERMS + term], to_fix(e, kEnergyScale));
+// A term's energy in fixed point and the index of its accumulator (-1: none
+// wanted).
+struct TermEnergy {
+  int key;
+  long long e;
+};
+__device__ __forceinline__ TermEnergy term_energy(const BondedArgs &a, int atom, int term, double e) {
+  if (!a.energy_mode) return TermEnergy{-1, 0};
+  return TermEnergy{a.atom_sys[atom] * PB2_NTERMS + term, to_fix(e, kEnergyScale)};
 }
 
 // Dihedral angle and its gradient w.r.t. the four atoms.
@@ -64,7 +69,7 @@ __device__ __forceinline__ int bonded_total(const BondedArgs &a) {
 // and impropers, CMAP, exception pairs, in that index order.  Inlined into
 // the bonded kernel; bonded_term_call keeps it out of line for the chain
 // pass, whose hot loop should not grow.
-static __device__ __forceinline__ void bonded_term(const BondedArgs &a, int t) {
+static __device__ __forceinline__ TermEnergy bonded_term(const BondedArgs &a, int t) {
   {
     int u = t;
     if (u < a.n_bond) {
@@ -75,9 +80,8 @@ static __device__ __forceinline__ void bonded_term(const BondedArgs &a, int t) {
       const double g = p.y * (r - p.x) / r;
       add_force(a, id.x, scale(d, -g));
       add_force(a, id.y, scale(d, g));
-      add_energy(a, id.x, u < a.n_bond_plain ? PB2_TERM_BOND : PB2_TERM_UREY_BRADLEY,
-                 0.5 * p.y * (r - p.x) * (r - p.x));
-      return;
+      return term_energy(a, id.x, u < a.n_bond_plain ? PB2_TERM_BOND : PB2_TERM_UREY_BRADLEY,
+                         0.5 * p.y * (r - p.x) * (r - p.x));
     }
     u -= a.n_bond;
     if (u < a.n_angle) {
@@ -101,8 +105,7 @@ static __device__ __forceinline__ void bonded_term(const BondedArgs &a, int t) {
       add_force(a, id.x, scale(gi, -1.0));
       add_force(a, id.y, {gi.x + gk.x, gi.y + gk.y, gi.z + gk.z});
       add_force(a, id.z, scale(gk, -1.0));
-      add_energy(a, id.x, PB2_TERM_ANGLE, 0.5 * p.y * (th - p.x) * (th - p.x));
-      return;
+      return term_energy(a, id.x, PB2_TERM_ANGLE, 0.5 * p.y * (th - p.x) * (th - p.x));
     }
     u -= a.n_angle;
     if (u < a.n_tors) {
@@ -129,8 +132,7 @@ static __device__ __forceinline__ void bonded_term(const BondedArgs &a, int t) {
       const int ids[4] = {id.x, id.y, id.z, id.w};
 #pragma unroll
       for (int c = 0; c < 4; ++c) add_force(a, ids[c], scale(g[c], -dedphi));
-      add_energy(a, id.x, term, e);
-      return;
+      return term_energy(a, id.x, term, e);
     }
     u -= a.n_tors;
     if (u < a.n_cmap) {
@@ -146,7 +148,7 @@ static __device__ __forceinline__ void bonded_term(const BondedArgs &a, int t) {
       const double delta = two_pi / G;
       const double pn = fmod(phi + two_pi, two_pi);
       const double sn = fmod(psi + two_pi, two_pi);
-      if (!(isfinite(pn) && isfinite(sn))) return;  // non-finite state: flagged by the integrator
+      if (!(isfinite(pn) && isfinite(sn))) return TermEnergy{-1, 0};  // non-finite state: flagged by the integrator
       int ia = (int)floor(pn / delta);
       int ib = (int)floor(sn / delta);
       ia = min(max(ia % G, 0), G - 1);
@@ -174,8 +176,7 @@ static __device__ __forceinline__ void bonded_term(const BondedArgs &a, int t) {
         add_force(a, row[k], scale(gphi[k], -ea));
         add_force(a, row[k + 1], scale(gpsi[k], -eb));
       }
-      add_energy(a, row[0], PB2_TERM_CMAP, e);
-      return;
+      return term_energy(a, row[0], PB2_TERM_CMAP, e);
     }
     u -= a.n_cmap;
     {  // explicit 1-4 exception pair (bonded.py:211-228)
@@ -198,7 +199,7 @@ static __device__ __forceinline__ void bonded_term(const BondedArgs &a, int t) {
       const double g = dedr * inv;
       add_force(a, id.x, scale(d, -g));
       add_force(a, id.y, scale(d, g));
-      add_energy(a, id.x, PB2_TERM_EXCEPTION, e);
+      return term_energy(a, id.x, PB2_TERM_EXCEPTION, e);
     }
   }
 }
