@@ -981,7 +981,7 @@ struct Timer {
 
 // Force kernels on the current posq; force accumulators must be zero (or
 // hold contributions to keep) and born_acc zero.  bonded_energy: also
-// accumulate the (FP64) bonded energies.  boxes_ready: the step kernel just
+// accumulate the (FP64) bonded energies.  boxes_ready: the launch before
 // wrote the block boxes (and ran the pair list's displacement test).
 static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_energy,
                                   bool boxes_ready = false) {
@@ -1084,16 +1084,12 @@ static cudaError_t enqueue_energy64(pb2_batch *b, cudaStream_t st) {
   return launch_energy64(1, ea, b->grid_e64[1], st);
 }
 
-static int fresh_forces(pb2_batch *b, cudaStream_t st, bool energy) {
+// Forces (and with energy set the FP64 energies) at the current positions,
+// or at the caller's device rows, which then become the positions.
+static int fresh_forces(pb2_batch *b, cudaStream_t st, bool energy, const double *rows = nullptr) {
   pb2_ctx *ctx = b->ctx;
-  const size_t nb = (size_t)b->n_total * sizeof(long long);
-  CUDA_TRY(ctx, cudaMemsetAsync(b->fx, 0, nb, st));
-  CUDA_TRY(ctx, cudaMemsetAsync(b->fy, 0, nb, st));
-  CUDA_TRY(ctx, cudaMemsetAsync(b->fz, 0, nb, st));
-  if (energy)
-    CUDA_TRY(ctx, cudaMemsetAsync(b->energy, 0, (size_t)b->n_sys * PB2_NTERMS * sizeof(long long), st));
-  CUDA_TRY(ctx, launch_posq(int_args(b, b->key_parity, 0), st));
-  CUDA_TRY(ctx, enqueue_forces(b, st, energy));
+  CUDA_TRY(ctx, launch_place(int_args(b, b->key_parity, 0), rows, energy ? b->energy : nullptr, st));
+  CUDA_TRY(ctx, enqueue_forces(b, st, energy, true));
   if (energy) CUDA_TRY(ctx, enqueue_energy64(b, st));
   b->forces_valid = true;
   return PB2_OK;
@@ -1115,15 +1111,9 @@ extern "C" int pb2_energy_forces_device(pb2_batch *b, const double *positions, d
   if (!b) return PB2_EINVAL;
   pb2_ctx *ctx = b->ctx;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t N = b->n_total;
-  if (positions) {
-    CUDA_TRY(ctx, cudaMemcpyAsync(b->stage, positions, 3 * N * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    CUDA_TRY(ctx, launch_rows_to_soa(b->stage, b->user, b->x, b->y, b->z, b->n_total, st));
-  }
-  int rc = fresh_forces(b, st, energies != nullptr);
+  int rc = fresh_forces(b, st, energies != nullptr, positions);
   if (rc) return rc;
-  if (energies) CUDA_TRY(ctx, launch_energies_to_double(b->energy, energies, b->n_sys, st));
-  if (forces) CUDA_TRY(ctx, launch_fix_to_rows(b->fx, b->fy, b->fz, b->user, forces, b->n_total, st));
+  CUDA_TRY(ctx, launch_results(b->fx, b->fy, b->fz, b->user, forces, b->n_total, b->energy, energies, b->n_sys, st));
   return PB2_OK;
 }
 

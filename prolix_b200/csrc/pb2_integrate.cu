@@ -466,6 +466,47 @@ __global__ void posq_kernel(const IntArgs a) {
   }
 }
 
+// The start of a force evaluation outside a step, one warp per 32-atom block:
+// positions from the caller's rows (rows NULL: the state's), the pair
+// kernels' float32 copy, the block's bounding box and the pair list's
+// displacement test, with the force and energy accumulators cleared.  One
+// launch where the copy, the conversion, four clears, the float32 copy and
+// the boxes took eight of 1.4 to 2 us each.
+__global__ void __launch_bounds__(128) place_kernel(const IntArgs a, const double *__restrict__ rows,
+                                                    long long *energy) {
+  const int lane = threadIdx.x & 31;
+  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+  if (energy)
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < a.n_sys * PB2_NTERMS; k += gridDim.x * blockDim.x)
+      energy[k] = 0;
+  bool moved = false;
+  for (int b = w; b < a.n_blocks; b += nw) {
+    const int4 info = a.blk_info[b];  // system, first atom, atoms
+    const SysInfo &S = a.sys[info.x];
+    const bool valid = lane < info.z;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (valid) {
+      const int i = info.y + lane;
+      const StepExtra e = step_extra(a, i);
+      double x, y, z;
+      if (rows) {
+        const double *r = rows + 3 * (size_t)a.user[i];
+        x = r[0]; y = r[1]; z = r[2];
+        a.x[i] = x; a.y[i] = y; a.z[i] = z;
+      } else {
+        x = a.x[i]; y = a.y[i]; z = a.z[i];
+      }
+      q = posq_of(x, y, z, make_double3(S.ox, S.oy, S.oz), e.charge);
+      a.posq[i] = q;
+      a.fx[i] = 0; a.fy[i] = 0; a.fz[i] = 0;
+      moved |= moved_past_half_skin(a, e, S, q);
+    }
+    block_box(a, b, lane, valid, q);
+  }
+  if (a.pl_ctl && __any_sync(kFull, moved) && lane == 0) atomicOr(&a.pl_ctl[PL_DIRTY], 1);
+}
+
 static int grid_for(int n) {
   int g = (n + 255) / 256;
   return g > 0 ? g : 1;
@@ -524,6 +565,11 @@ cudaError_t launch_center(const IntArgs &a, cudaStream_t st) {
   center_kernel<<<a.n_sys, kCenterThreads, 0, st>>>(a);
   return cudaGetLastError();
 }
+cudaError_t launch_place(const IntArgs &a, const double *rows, long long *energy, cudaStream_t st) {
+  place_kernel<<<(a.n_blocks + 3) / 4, 128, 0, st>>>(a, rows, energy);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_posq(const IntArgs &a, cudaStream_t st) {
   posq_kernel<<<grid_for(a.n_total), 256, 0, st>>>(a);
   return cudaGetLastError();

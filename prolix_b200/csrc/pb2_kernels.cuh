@@ -283,6 +283,9 @@ cudaError_t launch_noise_scale(const SysInfo *sys, const int32_t *atom_sys, cons
                                double *sigma, int n, cudaStream_t st);
 cudaError_t launch_init(const IntArgs &a, cudaStream_t st);
 cudaError_t launch_posq(const IntArgs &a, cudaStream_t st);
+// Positions in place for a force evaluation (rows: the caller's (n, 3)
+// positions, or NULL), boxes written, forces (and energies, unless NULL) cleared.
+cudaError_t launch_place(const IntArgs &a, const double *rows, long long *energy, cudaStream_t st);
 // Host transfers: `user` maps each batch atom to its row in the caller's
 // (n, 3) arrays.
 cudaError_t launch_rows_to_soa(const double *rows, const int32_t *user, double *x, double *y, double *z, int n,
@@ -299,6 +302,10 @@ cudaError_t launch_state_from_rows(const double *rows, const int32_t *user, doub
 cudaError_t launch_state_to_rows(const double *x, const double *y, const double *z, const double *px,
                                  const double *py, const double *pz, const long long *fx, const long long *fy,
                                  const long long *fz, const int32_t *user, double *rows, int n, cudaStream_t st);
+// An evaluation's results: forces in the caller's rows and energies in FP64
+// (either may be NULL), one launch.
+cudaError_t launch_results(const long long *fx, const long long *fy, const long long *fz, const int32_t *user,
+                           double *rows, int n, const long long *e, double *out, int n_sys, cudaStream_t st);
 cudaError_t launch_energies_to_double(const long long *e, double *out, int n_sys, cudaStream_t st);
 cudaError_t launch_snapshot(const double *x, const double *y, const double *z, const double *px,
                             const double *py, const double *pz, const double *mass, const long long *steps,

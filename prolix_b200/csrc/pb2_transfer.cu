@@ -38,15 +38,20 @@ __global__ void soa_to_rows(const double *__restrict__ x, const double *__restri
 
 // Fixed point -> FP64 is exact for |F| < 2^21 kcal/mol/A (|v| < 2^53), so a
 // get/set round trip restores the accumulators bit for bit.
+__device__ __forceinline__ void put_force_row(const long long *__restrict__ fx, const long long *__restrict__ fy,
+                                              const long long *__restrict__ fz, const int32_t *__restrict__ user,
+                                              double *rows, int i) {
+  double *r = rows + 3 * (size_t)user[i];
+  r[0] = (double)fx[i] * kForceInv;
+  r[1] = (double)fy[i] * kForceInv;
+  r[2] = (double)fz[i] * kForceInv;
+}
+
 __global__ void fix_to_rows(const long long *__restrict__ fx, const long long *__restrict__ fy,
                             const long long *__restrict__ fz, const int32_t *__restrict__ user, double *rows,
                             int n) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double *r = rows + 3 * (size_t)user[i];
-    r[0] = (double)fx[i] * kForceInv;
-    r[1] = (double)fy[i] * kForceInv;
-    r[2] = (double)fz[i] * kForceInv;
-  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    put_force_row(fx, fy, fz, user, rows, i);
 }
 
 __global__ void rows_to_fix(const double *__restrict__ rows, const int32_t *__restrict__ user, long long *fx,
@@ -75,16 +80,28 @@ __global__ void gather_systems(const SysInfo *sys, const int32_t *atom_sys, cons
 
 // Per-system term energies (2^-24 fixed point) to FP64, with the total
 // summed in term order.
-__global__ void energies_to_double(const long long *__restrict__ e, double *out, int n_sys) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_sys; s += gridDim.x * blockDim.x) {
-    double tot = 0.0;
-    for (int t = 0; t < PB2_TERM_TOTAL; ++t) {
-      const double v = (double)e[(size_t)s * PB2_NTERMS + t] * kEnergyInv;
-      out[(size_t)s * PB2_NTERMS + t] = v;
-      tot += v;
-    }
-    out[(size_t)s * PB2_NTERMS + PB2_TERM_TOTAL] = tot;
+__device__ __forceinline__ void put_energies(const long long *__restrict__ e, double *out, int s) {
+  double tot = 0.0;
+  for (int t = 0; t < PB2_TERM_TOTAL; ++t) {
+    const double v = (double)e[(size_t)s * PB2_NTERMS + t] * kEnergyInv;
+    out[(size_t)s * PB2_NTERMS + t] = v;
+    tot += v;
   }
+  out[(size_t)s * PB2_NTERMS + PB2_TERM_TOTAL] = tot;
+}
+
+__global__ void energies_to_double(const long long *__restrict__ e, double *out, int n_sys) {
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n_sys; s += gridDim.x * blockDim.x) put_energies(e, out, s);
+}
+
+__global__ void results_kernel(const long long *__restrict__ fx, const long long *__restrict__ fy,
+                               const long long *__restrict__ fz, const int32_t *__restrict__ user, double *rows,
+                               int n, const long long *__restrict__ e, double *out, int n_sys) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  if (out)
+    for (int s = t; s < n_sys; s += nt) put_energies(e, out, s);
+  if (rows)
+    for (int i = t; i < n; i += nt) put_force_row(fx, fy, fz, user, rows, i);
 }
 
 // Trajectory frame: float32 positions and velocities (p / m), (n, 3) each
@@ -182,6 +199,13 @@ cudaError_t launch_gather_systems(const SysInfo *sys, const int32_t *atom_sys, c
   if (n <= 0) return cudaSuccess;
   gather_systems<<<grid_for(n), 256, 0, st>>>(sys, atom_sys, perm, user, devidx, (const unsigned long long *)src,
                                               (unsigned long long *)dst, n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_results(const long long *fx, const long long *fy, const long long *fz, const int32_t *user,
+                           double *rows, int n, const long long *e, double *out, int n_sys, cudaStream_t st) {
+  if (!rows && !out) return cudaSuccess;
+  results_kernel<<<grid_for(rows ? n : n_sys), 256, 0, st>>>(fx, fy, fz, user, rows, n, e, out, n_sys);
   return cudaGetLastError();
 }
 
