@@ -34,7 +34,7 @@ from pathlib import Path
 
 import numpy as np
 
-CANDIDATES = (2, 4, 8, 16, 32)
+CANDIDATES = (1, 2, 4, 8, 16, 32)
 
 
 def cache_path() -> Path:

@@ -223,14 +223,32 @@ static void spatial_order(const double *pos, int n, std::vector<int> &ord) {
   for (int a = 0; a < n; a += 32) std::sort(ord.begin() + a, ord.begin() + std::min(n, a + 32));
 }
 
-// Work items of the two-i-block force kernel: even i-blocks ib (with ib + 1)
-// against j-blocks [j0, j1), j0 >= ib.
+// Work items of the two-i-block kernels: even i-blocks ib (with ib + 1)
+// against j-blocks [j0, j1), j0 >= ib, of at most seg tiles, longest first.
+// Where few items are shorter than seg by nature (long rows), a sixth of each
+// row's tiles are items of their own: handed out last, they fill the end of
+// the pass, where the last warps' whole segments would leave the others idle
+// (20,000 atoms, all pairs, seg 4: 825 -> 806 us per step; a ragged batch has
+// its rows' short remainders for that, and 15 % more single tiles cost it 1 %).
 static std::vector<TileItem> build_items2(const std::vector<SysInfo> &sinfo, int seg) {
+  long long tiles = 0, rest = 0;  // all, and in the rows' last, shorter items
+  for (const SysInfo &S : sinfo)
+    for (int ib = 0; ib < S.nblk; ib += 2) {
+      tiles += S.nblk - ib;
+      rest += (S.nblk - ib) % seg;
+    }
+  const bool singles = 20 * rest < tiles;
   std::vector<TileItem> items;
   for (int s = 0; s < (int)sinfo.size(); ++s) {
     const int nblk = sinfo[s].nblk;
-    for (int ib = 0; ib < nblk; ib += 2)
-      for (int j0 = ib; j0 < nblk; j0 += seg) items.push_back(TileItem{s, ib, j0, std::min(j0 + seg, nblk)});
+    for (int ib = 0; ib < nblk; ib += 2) {
+      const int whole = singles ? ib + (nblk - ib) * 5 / 6 / seg * seg : nblk;  // seg tiles per item up to here
+      for (int j0 = ib; j0 < nblk;) {
+        const int j1 = std::min(j0 + (j0 < whole ? seg : 1), nblk);
+        items.push_back(TileItem{s, ib, j0, j1});
+        j0 = j1;
+      }
+    }
   }
   std::stable_sort(items.begin(), items.end(), [](const TileItem &p, const TileItem &q) {
     return (p.jb1 - p.jb0) > (q.jb1 - q.jb0);
@@ -476,12 +494,16 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   b->ctx = ctx;
   b->params = *params;
   if (b->params.tile_segment <= 0) {
-    // default work-item length: the longest (8, 4, 2 or 1 j-blocks) that
-    // still gives every resident warp of the force pass a few items, so a
-    // small batch spreads over the whole GPU
+    // default work-item length: the longest (6, 4, 2 or 1 j-blocks) that still
+    // gives every resident warp of the force pass a few items, so a small
+    // batch spreads over the whole GPU; single tiles with a pair list, whose
+    // items come in no order.  us per step with 8, 6, 4, 2, 1: a ragged batch
+    // of 256 systems 1308, 1308, 1325, 1346, 1398; 20,000 atoms 817, 807, 806,
+    // 826, 891; the same at 20 A 264, 260, 232, 201, 191
     const long long want = 4LL * ctx->sm_count * 16;
     int seg = 1;
-    for (int cand : {8, 4, 2}) {
+    for (int cand : {6, 4, 2}) {
+      if (params->cutoff > 0.0) break;
       long long items = 0;
       for (int s = 0; s < n_systems; ++s) {
         const int nb = (systems[s].n_atoms + 31) / 32;
@@ -826,7 +848,11 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
       finite = finite && gb_cut_mode;
       reach = std::max(reach, std::max(gb_cut, born_cut));
     }
-    b->pl_on = finite && (direct || gbt);
+    // (it saves less than its update costs where no system has many blocks:
+    // us per step with and without at 1,200 atoms, 20 A: 30.7, 29.0; 2,500,
+    // 9 A: 47.9, 51.2; 4,000, 12 A: 56.6, 59.7)
+    const bool many = std::any_of(sinfo.begin(), sinfo.end(), [](const SysInfo &S) { return S.nblk >= 64; });
+    b->pl_on = finite && (direct || gbt) && many;
     b->pl_reach2 = (float)((reach + params->skin) * (reach + params->skin));
   }
   b->q64 = D.alloc<double>(N);
