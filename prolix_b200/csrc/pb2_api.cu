@@ -305,12 +305,17 @@ static void set_force4_grid(pb2_batch *b) {
   b->grid4 = std::max(1, std::min(cap, (b->n_items4 + w - 1) / w));
 }
 
-// Grid of pair pass p for its block shape: one resident wave (warps take
-// items dynamically), no more warps than items.
+// Grid of pair pass p for its block shape: one resident wave, no more thread
+// blocks than units of work (items; for the chain pass the bonded chunks
+// too, for the descreening pass the finalize chunks), of which few spread
+// over the SMs.
 static void set_pair_grid(pb2_batch *b, int p) {
   const int cap = tile_kernel_occupancy(p, b->cut, b->shape[p]) * b->ctx->sm_count;
-  const int w = tile_kernel_warps(p, b->shape[p]);
-  b->grid_pair[p] = std::max(1, std::min(cap, (b->n_items2 + w - 1) / w));
+  const BondedArgs &ba = b->bonded;
+  const int bonded = ba.n_bond + ba.n_angle + ba.n_tors + ba.n_cmap + ba.n_exc;
+  const int chunks = (bonded + kBondedChunk - 1) / kBondedChunk;
+  const int units = b->n_items2 + (p == PASS_CHAIN ? chunks : p == PASS_BORN ? b->n_blocks : 0);
+  b->grid_pair[p] = std::max(1, std::min(cap, units));
 }
 
 // (Re)build the pair kernels' two-i-block work list and their grids (one

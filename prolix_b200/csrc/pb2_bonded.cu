@@ -26,6 +26,8 @@ namespace pb2 {
 // once: the terms of a kind all meet at one address, and 80,000 atomics on
 // four addresses took 38 of the kernel's 43 us at N = 20,000.
 __global__ void bonded_kernel(const BondedArgs a) {
+  // The terms read positions, which the launch before (a pair pass) does not
+  // write, and add to accumulators: they need not wait for it.
   const int total = bonded_total(a);
   const int lane = threadIdx.x & 31;
   for (int t0 = blockIdx.x * blockDim.x + threadIdx.x - lane; t0 < total; t0 += gridDim.x * blockDim.x) {
@@ -41,6 +43,7 @@ __global__ void bonded_kernel(const BondedArgs a) {
       if (v.key >= 0 && (!same || lane == 0)) atomic_add_fix(&a.energy[v.key], v.e);
     }
   }
+  pdl_wait();
 }
 
 cudaError_t launch_bonded(const BondedArgs &a, int grid_cap, cudaStream_t st) {
@@ -48,8 +51,7 @@ cudaError_t launch_bonded(const BondedArgs &a, int grid_cap, cudaStream_t st) {
   if (total <= 0) return cudaSuccess;
   int grid = (total + 255) / 256;
   if (grid > grid_cap) grid = grid_cap;
-  bonded_kernel<<<grid, 256, 0, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(bonded_kernel, grid, 256, st, a);
 }
 
 }  // namespace pb2

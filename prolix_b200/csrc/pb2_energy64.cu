@@ -290,6 +290,8 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
   M.use_coul = (a.terms & PB2_USE_COULOMB) != 0;
   const bool all_terms = M.use_gb && M.use_lj && M.use_coul;
   const uint32_t diag_mask = lane == 31 ? 0u : (0xffffffffu << (lane + 1));
+  pdl_wait();
+  pdl_trigger();
   for (int it = wl * (int)gridDim.x + (int)blockIdx.x; it < a.n_items;) {
     const TileItem item = a.items[it];
     const ItemRange R = item_range(item);
@@ -443,6 +445,8 @@ __device__ __forceinline__ long long warp_sum_ll(long long v) {
 __global__ void __launch_bounds__(128) finalize64_kernel(const Energy64Args a) {
   const int lane = threadIdx.x & 31;
   const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+  pdl_wait();
+  pdl_trigger();
   for (int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); b < a.n_blocks; b += nw) {
     const int s = a.blk_sys[b];
     const SysInfo &S = a.sys[s];
@@ -469,15 +473,12 @@ __global__ void __launch_bounds__(128) finalize64_kernel(const Energy64Args a) {
 
 cudaError_t launch_finalize64(const Energy64Args &a, cudaStream_t st) {
   if (a.n_blocks <= 0) return cudaSuccess;
-  finalize64_kernel<<<(a.n_blocks + 3) / 4, 128, 0, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(finalize64_kernel, (a.n_blocks + 3) / 4, 128, st, a);
 }
 
 cudaError_t launch_energy64(int pass, const Energy64Args &a, int grid, cudaStream_t st) {
   if (a.n_items <= 0) return cudaSuccess;
-  if (pass == 0) energy64_kernel<0><<<grid, kE64Threads, 0, st>>>(a);
-  else energy64_kernel<1><<<grid, kE64Threads, 0, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(pass == 0 ? energy64_kernel<0> : energy64_kernel<1>, grid, kE64Threads, st, a);
 }
 
 int energy64_occupancy(int pass) {

@@ -131,21 +131,35 @@ constexpr int kStepWarps = 4;  // warps per thread block of the plain step
 
 // Block info (system, first atom, atoms): lanes past the block's last atom
 // copy its first atom (never used).
-__device__ __forceinline__ void issue_block(const IntArgs &a, int4 info, int lane, StepIn &B) {
+__device__ __forceinline__ void issue_state(const IntArgs &a, int4 info, int lane, StepIn &B) {
   const int i = info.y + (lane < info.z ? lane : 0);
   cp_async8(&B.x[0][lane], a.x + i); cp_async8(&B.x[1][lane], a.y + i); cp_async8(&B.x[2][lane], a.z + i);
   cp_async8(&B.p[0][lane], a.px + i); cp_async8(&B.p[1][lane], a.py + i); cp_async8(&B.p[2][lane], a.pz + i);
-  cp_async8(&B.f[0][lane], a.fx + i); cp_async8(&B.f[1][lane], a.fy + i); cp_async8(&B.f[2][lane], a.fz + i);
   cp_async8(&B.m[lane], a.mass + i); cp_async8(&B.sg[lane], a.sigma + i); cp_async8(&B.q[lane], a.charge + i);
   cp_async4(&B.user[lane], a.user + i);
+}
+__device__ __forceinline__ void issue_force(const IntArgs &a, int4 info, int lane, StepIn &B) {
+  const int i = info.y + (lane < info.z ? lane : 0);
+  cp_async8(&B.f[0][lane], a.fx + i); cp_async8(&B.f[1][lane], a.fy + i); cp_async8(&B.f[2][lane], a.fz + i);
+}
+
+// The atom's three normals of this step; rnd: its index in the caller's
+// order, which its noise follows.
+__device__ __forceinline__ float3 step_noise(const IntArgs &a, int s, const SysInfo &S, int rnd) {
+  const uint4 sp = reinterpret_cast<const uint4 *>(a.splits)[(size_t)a.parity * a.n_sys + s];
+  const uint32_t sub[2] = {sp.z, sp.w};
+  const uint32_t count = 3u * (uint32_t)S.n, k = 3u * (uint32_t)rnd;
+  const bool part = a.partitionable != 0;
+  return make_float3(normal_from_bits(random_bits32(sub, k, count, part)),
+                     normal_from_bits(random_bits32(sub, k + 1u, count, part)),
+                     normal_from_bits(random_bits32(sub, k + 2u, count, part)));
 }
 
 // One atom's plain BAOAB step from its copied inputs; returns the float32
 // position it wrote.
 __device__ __forceinline__ float4 step_atom(const IntArgs &a, int i, int s, const SysInfo &S, const StepIn &B,
-                                            int lane) {
+                                            float3 noise, int lane) {
   const int loc = i - S.off;
-  const int rnd = B.user[lane] - S.off;  // the atom's index in the caller's order: its noise
   const double h = S.half_dt;
   const double m = B.m[lane];
   const double rm = __drcp_rn(m);  // p / m = div_by(p, m, rm), correctly rounded
@@ -155,17 +169,14 @@ __device__ __forceinline__ float4 step_atom(const IntArgs &a, int i, int s, cons
   a.fx[i] = 0; a.fy[i] = 0; a.fz[i] = 0;
   double p[3] = {B.p[0][lane], B.p[1][lane], B.p[2][lane]};
   double x[3] = {B.x[0][lane], B.x[1][lane], B.x[2][lane]};
-  const uint4 sp = reinterpret_cast<const uint4 *>(a.splits)[(size_t)a.parity * a.n_sys + s];
-  const uint32_t knew[2] = {sp.x, sp.y}, sub[2] = {sp.z, sp.w};
-  const uint32_t count = 3u * (uint32_t)S.n;
   const double c1 = S.c1, sg = B.sg[lane];
+  const float xi3[3] = {noise.x, noise.y, noise.z};
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     if (a.finish_prev) p[c] = __dadd_rn(p[c], __dmul_rn(h, f[c]));
     p[c] = __dadd_rn(p[c], __dmul_rn(h, f[c]));
     x[c] = __dadd_rn(x[c], __dmul_rn(h, div_by(p[c], m, rm)));
-    const float xi = normal_from_bits(random_bits32(sub, 3u * (uint32_t)rnd + c, count, a.partitionable != 0));
-    p[c] = __dadd_rn(__dmul_rn(c1, p[c]), __dmul_rn(sg, (double)xi));
+    p[c] = __dadd_rn(__dmul_rn(c1, p[c]), __dmul_rn(sg, (double)xi3[c]));
     x[c] = __dadd_rn(x[c], __dmul_rn(h, div_by(p[c], m, rm)));
   }
   a.px[i] = p[0]; a.py[i] = p[1]; a.pz[i] = p[2];
@@ -175,7 +186,11 @@ __device__ __forceinline__ float4 step_atom(const IntArgs &a, int i, int s, cons
   if (!(isfinite(x[0]) && isfinite(x[1]) && isfinite(x[2]) && isfinite(p[0]) &&
         isfinite(p[1]) && isfinite(p[2])))
     atomicOr(&a.status[s], (uint32_t)PB2_STATUS_NONFINITE);
-  if (loc == 0) advance_key(a, s, knew);
+  if (loc == 0) {
+    const uint4 sp = reinterpret_cast<const uint4 *>(a.splits)[(size_t)a.parity * a.n_sys + s];
+    const uint32_t knew[2] = {sp.x, sp.y};
+    advance_key(a, s, knew);
+  }
   return q;
 }
 
@@ -189,12 +204,32 @@ __global__ void __launch_bounds__(32 * kStepWarps, 6) step_kernel(const IntArgs 
   bool moved = false;
   const int4 none = make_int4(0, 0, 0, 0);
   int4 info = b < a.n_blocks ? a.blk_info[b] : none;
-  if (b < a.n_blocks) issue_block(a, info, lane, s_in[wl][0]);
+  // After a step of the same chunk the launch before (a force kernel) wrote
+  // only forces, and the state is from before it: the first block's state is
+  // copied and its noise drawn while that launch still runs.
+  const bool early = a.finish_prev != 0;
+  if (!early) pdl_wait();
+  if (b < a.n_blocks) issue_state(a, info, lane, s_in[wl][0]);
+  cp_async_commit();
+  float3 noise0 = make_float3(0.f, 0.f, 0.f);
+  if (early) {
+    cp_async_wait<0>();
+    if (lane < info.z) {
+      const SysInfo &S = a.sys[info.x];
+      noise0 = step_noise(a, info.x, S, s_in[wl][0].user[lane] - S.off);
+    }
+    pdl_wait();
+  }
+  pdl_trigger();
+  if (b < a.n_blocks) issue_force(a, info, lane, s_in[wl][0]);
   cp_async_commit();
   int4 info_next = b + nw < a.n_blocks ? a.blk_info[b + nw] : none;
   for (int it = 0; b < a.n_blocks; b += nw, ++it) {
     const int bn = b + nw;
-    if (bn < a.n_blocks) issue_block(a, info_next, lane, s_in[wl][(it + 1) & 1]);
+    if (bn < a.n_blocks) {
+      issue_state(a, info_next, lane, s_in[wl][(it + 1) & 1]);
+      issue_force(a, info_next, lane, s_in[wl][(it + 1) & 1]);
+    }
     cp_async_commit();
     const int4 cur = info;
     info = info_next;
@@ -208,7 +243,9 @@ __global__ void __launch_bounds__(32 * kStepWarps, 6) step_kernel(const IntArgs 
       if (valid) {
         StepExtra e;  // the charge comes from the copied inputs
         e.ref = a.pl_ref ? a.pl_ref[cur.y + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-        q = step_atom(a, cur.y + lane, s, S, s_in[wl][it & 1], lane);
+        float3 noise = noise0;
+        if (!early || it > 0) noise = step_noise(a, s, S, s_in[wl][it & 1].user[lane] - S.off);
+        q = step_atom(a, cur.y + lane, s, S, s_in[wl][it & 1], noise, lane);
         moved |= moved_past_half_skin(a, e, S, q);
       }
       block_box(a, b, lane, valid, q);
@@ -330,6 +367,8 @@ __device__ __forceinline__ float4 step_guarded_atom(const IntArgs &a, int i, int
 }
 
 __global__ void __launch_bounds__(256, 4) step_guarded_kernel(const IntArgs a) {
+  pdl_wait();
+  pdl_trigger();
   const bool cap_open = a.finish_prev || *a.guard_end;
   const int lane = threadIdx.x & 31;
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -354,6 +393,7 @@ __global__ void __launch_bounds__(256, 4) step_guarded_kernel(const IntArgs a) {
 }
 
 __global__ void finish_guarded_kernel(const IntArgs a) {
+  pdl_wait();
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.guard_end = 1;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
     const int s = a.atom_sys[i];
@@ -375,6 +415,7 @@ __global__ void finish_guarded_kernel(const IntArgs a) {
 }
 
 __global__ void finish_kernel(const IntArgs a) {
+  pdl_wait();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
     const int s = a.atom_sys[i];
     if (a.retired[s]) continue;
@@ -477,6 +518,8 @@ __global__ void __launch_bounds__(128) place_kernel(const IntArgs a, const doubl
   const int lane = threadIdx.x & 31;
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+  pdl_wait();
+  pdl_trigger();
   if (energy)
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < a.n_sys * PB2_NTERMS; k += gridDim.x * blockDim.x)
       energy[k] = 0;
@@ -536,17 +579,11 @@ cudaError_t launch_step(const IntArgs &a, cudaStream_t st) {
   const int grid = (a.n_blocks + 7) / 8;  // 8 warps, one 32-atom block each
   if (grid <= 0) return cudaSuccess;
   if (guarded(a))
-    step_guarded_kernel<<<grid, 256, 0, st>>>(a);
-  else
-    step_kernel<<<step_grid(a.n_blocks), 32 * kStepWarps, 0, st>>>(a);
-  return cudaGetLastError();
+    return launch_after(step_guarded_kernel, grid, 256, st, a);
+  return launch_after(step_kernel, step_grid(a.n_blocks), 32 * kStepWarps, st, a);
 }
 cudaError_t launch_finish(const IntArgs &a, cudaStream_t st) {
-  if (guarded(a))
-    finish_guarded_kernel<<<grid_for(a.n_total), 256, 0, st>>>(a);
-  else
-    finish_kernel<<<grid_for(a.n_total), 256, 0, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(guarded(a) ? finish_guarded_kernel : finish_kernel, grid_for(a.n_total), 256, st, a);
 }
 cudaError_t launch_key_splits(const IntArgs &a, cudaStream_t st) {
   key_splits_kernel<<<(a.n_sys + 255) / 256, 256, 0, st>>>(a);
@@ -566,8 +603,7 @@ cudaError_t launch_center(const IntArgs &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 cudaError_t launch_place(const IntArgs &a, const double *rows, long long *energy, cudaStream_t st) {
-  place_kernel<<<(a.n_blocks + 3) / 4, 128, 0, st>>>(a, rows, energy);
-  return cudaGetLastError();
+  return launch_after(place_kernel, (a.n_blocks + 3) / 4, 128, st, a, rows, energy);
 }
 
 cudaError_t launch_posq(const IntArgs &a, cudaStream_t st) {

@@ -92,6 +92,8 @@ __device__ __forceinline__ void block_sum3(double &v0, double &v1, double &v2) {
 // ----------------------------------------------------------- steepest descent
 
 __global__ void min_sd_kernel(const MinArgs a) {
+  pdl_wait();
+  pdl_trigger();
   const double dt = a.par[kMinSdDt], max_dx = a.par[kMinMaxDx];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
     double f[3];
@@ -153,6 +155,8 @@ __global__ void min_fire_init_kernel(const MinArgs a) {
 // Start of an iteration: RMS of the state force; keep the positions if it is
 // the lowest so far.
 __global__ void min_fire_begin_kernel(const MinArgs a) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ int better;
   const size_t N = a.n_total;
   for (int s = blockIdx.x; s < a.n_sys; s += gridDim.x) {
@@ -179,6 +183,8 @@ __global__ void min_fire_begin_kernel(const MinArgs a) {
 // cap.  With a force cap (prolix simulate.py:613-621) the state force of
 // each atom is scaled to at most that norm for this kick.
 __global__ void min_fire_drift_kernel(const MinArgs a) {
+  pdl_wait();
+  pdl_trigger();
   const size_t N = a.n_total;
   const double cap = a.par[kMinForceCap];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
@@ -202,6 +208,8 @@ __global__ void min_fire_drift_kernel(const MinArgs a) {
 // Second half kick with the new force, FIRE mixing and time-step control,
 // then the displacement cap.
 __global__ void min_fire_mix_kernel(const MinArgs a) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ double mix_f, mix_p;
   __shared__ int zero_p;
   const size_t N = a.n_total;
@@ -473,12 +481,12 @@ cudaError_t launch_min(int op, const MinArgs &a, double *out, cudaStream_t st) {
   if (a.n_total <= 0) return cudaSuccess;
   const int ga = atom_grid(a.n_total), gs = a.n_sys;
   switch (op) {
-    case kMinOpSd: min_sd_kernel<<<ga, kMinThreads, 0, st>>>(a); break;
+    case kMinOpSd: return launch_after(min_sd_kernel, ga, kMinThreads, st, a);
     case kMinOpRollback: min_rollback_kernel<<<gs, kMinThreads, 0, st>>>(a); break;
     case kMinOpFireInit: min_fire_init_kernel<<<ga, kMinThreads, 0, st>>>(a); break;
-    case kMinOpFireBegin: min_fire_begin_kernel<<<gs, kMinThreads, 0, st>>>(a); break;
-    case kMinOpFireDrift: min_fire_drift_kernel<<<ga, kMinThreads, 0, st>>>(a); break;
-    case kMinOpFireMix: min_fire_mix_kernel<<<gs, kMinThreads, 0, st>>>(a); break;
+    case kMinOpFireBegin: return launch_after(min_fire_begin_kernel, gs, kMinThreads, st, a);
+    case kMinOpFireDrift: return launch_after(min_fire_drift_kernel, ga, kMinThreads, st, a);
+    case kMinOpFireMix: return launch_after(min_fire_mix_kernel, gs, kMinThreads, st, a);
     case kMinOpTakeBest: min_take_best_kernel<<<ga, kMinThreads, 0, st>>>(a); break;
     case kMinOpRms: min_rms_kernel<<<gs, kMinThreads, 0, st>>>(a, out); break;
     default: return cudaErrorInvalidValue;

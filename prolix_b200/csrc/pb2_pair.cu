@@ -628,6 +628,8 @@ __device__ __noinline__ void finalize_chunk(const PairArgs &a, int c, const int3
 }
 
 __global__ void born_finalize(const FinalizeArgs a) {
+  pdl_wait();
+  pdl_trigger();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
     finalize_atom(a, i, a.sys[a.atom_sys[i]]);
   }
@@ -673,6 +675,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   const uint32_t diag_mask = lane == 31 ? 0u : (0xffffffffu << (lane + 1));
   const float bscale = PASS == PASS_BORN ? (float)kBornScale : (float)kForceScale;
 
+  pdl_wait();
   // a cutoff run with a pair list takes its items (and each item's j-blocks)
   // from the list; otherwise items are contiguous j-block ranges
   const bool plm = CUT && a.pl_ctl != nullptr;
@@ -685,10 +688,22 @@ __global__ void __launch_bounds__(THREADS, MINB)
     n_items = a.pl_ctl[PL_COUNT0 + cur];
     if (sys_items) sys_items = cur ? a.pl_sys_items1 : a.pl_sys_items0;
   }
-  for (;;) {
-    int it = 0;
-    if (lane == 0) it = atomicAdd(&a.sched[0], 1);
-    it = __shfl_sync(kFull, it, 0);
+  // A pass of one wave lets the next launch's blocks start beside it; a
+  // longer one does not (a ragged batch's step 1,330 us, with it 1,353).
+  if (n_items <= nwarps) pdl_trigger();
+  // Each warp starts with an item of its own, consecutive ones on different
+  // SMs (few items then spread over the chip, and no warp waits for the
+  // counter first), and takes further ones from the counter.  A fused
+  // finalize waits for items: there every item comes from the counter, so
+  // that each one waited for was taken by a running warp.
+  const bool counted = PASS == PASS_BORN && sys_items;
+  const int base = counted ? 0 : nwarps;
+  int it = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+  for (bool own = !counted;; own = false) {
+    if (!own) {
+      if (lane == 0) it = base + atomicAdd(&a.sched[0], 1);
+      it = __shfl_sync(kFull, it, 0);
+    }
     if (it >= n_items) {
       if constexpr (PASS == PASS_BORN) {
         // tail work: the Born radii of one 32-atom block, once its system's
@@ -907,6 +922,8 @@ __global__ void __launch_bounds__(THREADS, MINB) force4_kernel(const __grid_cons
   long long *ps = &s_ps[threadIdx.x >> 5][0][lane];
   const uint32_t diag_mask = lane == 31 ? 0u : (0xffffffffu << (lane + 1));
   const float bscale = (float)kForceScale;
+  pdl_wait();
+  pdl_trigger();
   const int n_items = a.item_count ? *a.item_count : a.n_items;
   for (;;) {
     int it = 0;
@@ -1062,6 +1079,8 @@ __global__ void bbox_kernel(const SysInfo *sys, const int32_t *blk_sys, const fl
   const int lane = threadIdx.x & 31;
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nw = (int)((gridDim.x * blockDim.x) >> 5);
+  pdl_wait();
+  pdl_trigger();
   bool moved = false;  // this lane saw an atom beyond skin / 2 of the pair list's reference
   for (int b = w; b < n_blocks; b += nw) {
     const SysInfo &S = sys[blk_sys[b]];
@@ -1112,7 +1131,7 @@ constexpr Shape kShapes[3][kShapesPerPass] = {
 template <int PASS, bool CUT, bool ALL, int SH>
 static void launch_one(const PairArgs &a, int grid, cudaStream_t st) {
   constexpr Shape sh = kShapes[PASS][SH];
-  tile2_kernel<PASS, CUT, ALL, sh.threads, sh.minb><<<grid, sh.threads, 0, st>>>(a);
+  launch_after(tile2_kernel<PASS, CUT, ALL, sh.threads, sh.minb>, grid, sh.threads, st, a);
 }
 
 template <int PASS, bool CUT, bool ALL>
@@ -1153,15 +1172,13 @@ cudaError_t launch_bbox(const SysInfo *sys, const int32_t *blk_sys, const float4
                         int n_blocks, cudaStream_t st, const float4 *pl_ref, int32_t *pl_ctl) {
   if (n_blocks <= 0) return cudaSuccess;
   const int grid = (n_blocks + 7) / 8;
-  bbox_kernel<<<grid, 256, 0, st>>>(sys, blk_sys, posq, bbox, n_blocks, pl_ref, pl_ctl);
-  return cudaGetLastError();
+  return launch_after(bbox_kernel, grid, 256, st, sys, blk_sys, posq, bbox, n_blocks, pl_ref, pl_ctl);
 }
 
 cudaError_t launch_born_finalize(const FinalizeArgs &a, cudaStream_t st) {
   if (a.n_total <= 0) return cudaSuccess;
   const int grid = (a.n_total + 255) / 256;
-  born_finalize<<<grid, 256, 0, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(born_finalize, grid, 256, st, a);
 }
 
 template <int PASS, bool CUT, bool ALL, int SH>
@@ -1189,7 +1206,7 @@ constexpr Shape kShapes4[kShapesPerPass] = {{128, 3}, {128, 2}, {64, 5}};
 template <bool CUT, bool ALL, int SH>
 static void launch_force4_one(const PairArgs &a, int grid, cudaStream_t st) {
   constexpr Shape sh = kShapes4[SH];
-  force4_kernel<CUT, ALL, sh.threads, sh.minb><<<grid, sh.threads, 0, st>>>(a);
+  launch_after(force4_kernel<CUT, ALL, sh.threads, sh.minb>, grid, sh.threads, st, a);
 }
 template <bool CUT, bool ALL>
 static void launch_force4_shaped(const PairArgs &a, int grid, int shape, cudaStream_t st) {

@@ -38,6 +38,8 @@ __device__ __forceinline__ float pl_box_dist2(const float4 *bbox, int a, int b) 
 
 // One warp per list row (a pair of i-blocks).
 __global__ void pl_update_kernel(const PlArgs a) {
+  pdl_wait();
+  pdl_trigger();
   if (a.ctl[PL_DIRTY] == 0) return;  // the whole grid sees the same flag
   const int lane = threadIdx.x & 31;
   const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -104,8 +106,7 @@ __global__ void pl_update_kernel(const PlArgs a) {
 
 cudaError_t launch_pl_update(const PlArgs &a, int grid, cudaStream_t st) {
   if (a.n_rows <= 0) return cudaSuccess;
-  pl_update_kernel<<<grid, 256, 0, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(pl_update_kernel, grid, 256, st, a);
 }
 
 // Retire a system and re-list the live work items: an ordered compaction

@@ -98,6 +98,7 @@ __global__ void results_kernel(const long long *__restrict__ fx, const long long
                                const long long *__restrict__ fz, const int32_t *__restrict__ user, double *rows,
                                int n, const long long *__restrict__ e, double *out, int n_sys) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  pdl_wait();
   if (out)
     for (int s = t; s < n_sys; s += nt) put_energies(e, out, s);
   if (rows)
@@ -205,8 +206,7 @@ cudaError_t launch_gather_systems(const SysInfo *sys, const int32_t *atom_sys, c
 cudaError_t launch_results(const long long *fx, const long long *fy, const long long *fz, const int32_t *user,
                            double *rows, int n, const long long *e, double *out, int n_sys, cudaStream_t st) {
   if (!rows && !out) return cudaSuccess;
-  results_kernel<<<grid_for(rows ? n : n_sys), 256, 0, st>>>(fx, fy, fz, user, rows, n, e, out, n_sys);
-  return cudaGetLastError();
+  return launch_after(results_kernel, grid_for(rows ? n : n_sys), 256, st, fx, fy, fz, user, rows, n, e, out, n_sys);
 }
 
 cudaError_t launch_energies_to_double(const long long *e, double *out, int n_sys, cudaStream_t st) {
