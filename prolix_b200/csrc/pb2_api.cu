@@ -82,6 +82,7 @@ static PairArgs pair_args(pb2_batch *b) {
   a.bbox = b->bbox;
   a.cut = b->cut ? 1 : 0;
   a.sched = b->sched;
+  a.early = 0;
   a.born_acc = b->born_acc;
   a.dedb_acc = b->dedb_acc;
   a.fx = b->fx;
@@ -318,6 +319,24 @@ static void set_pair_grid(pb2_batch *b, int p) {
   b->grid_pair[p] = std::max(1, std::min(cap, units));
 }
 
+// Teams (a thread block of 8 or 4 warps per tile) for a batch of so few tiles
+// that with one warp each the chip waits for single warps' steps.  The lines
+// lie where the step times cross (us per step, one system, all pairs; none /
+// 8 warps / 4 warps): 896 atoms, 210 tiles 36.9 / 22.5 / 24.9; 1,200, 380
+// tiles 38.8 / 31.5 / 28.0; 1,500, 576 tiles 40.1 / 36.0 / 30.6; 1,800, 841
+// tiles 40.1 / 45.7 / 41.8.
+static void set_team(pb2_batch *b, int seg) {
+  const int n = b->n_items2;
+  b->team = seg != 1 ? 0 : n <= 296 ? 8 : n <= 640 ? 4 : 0;
+  if (!b->team) return;
+  const BondedArgs &ba = b->bonded;
+  const int bonded = ba.n_bond + ba.n_angle + ba.n_tors + ba.n_cmap + ba.n_exc;
+  for (int p = 0; p < 3; ++p) {
+    const int units = n + (p == PASS_CHAIN ? (bonded + kBondedChunk * b->team - 1) / (kBondedChunk * b->team) : 0);
+    b->grid_team[p] = std::max(1, std::min(team_occupancy(p, b->team, b->cut) * b->ctx->sm_count, units));
+  }
+}
+
 // (Re)build the pair kernels' two-i-block work list and their grids (one
 // resident wave each; warps take items dynamically).  The kernels read the
 // live list: the full one without the items of retired systems.
@@ -367,6 +386,7 @@ static int setup_items2(pb2_batch *b, int seg) {
   CUDA_TRY(ctx, cudaMemcpy(b->sys_items, per_sys.data(), per_sys.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
   b->sys_items_host = per_sys;
   for (int p = 0; p < 3; ++p) set_pair_grid(b, p);
+  set_team(b, seg);
   set_force4_grid(b);
   return PB2_OK;
 }
@@ -1010,6 +1030,13 @@ struct Timer {
   }
 };
 
+// A pair pass: by teams where the batch has few tiles (not with the fused
+// finalize, which is tail work of the one-warp kernel).
+static cudaError_t enqueue_pass(pb2_batch *b, int pass, const PairArgs &a, cudaStream_t st) {
+  if (b->team && !a.sys_items) return launch_team(pass, b->team, a, b->grid_team[pass], st);
+  return launch_tiles(pass, a, b->grid_pair[pass], b->shape[pass], st);
+}
+
 // Force kernels on the current posq; force accumulators must be zero (or
 // hold contributions to keep) and born_acc zero.  bonded_energy: also
 // accumulate the (FP64) bonded energies.  boxes_ready: the launch before
@@ -1051,12 +1078,12 @@ static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_ene
       pb.sys_items = b->sys_items;
       pb.fin = fa;
     }
-    if ((e = tm(kTimBorn, [&] { return launch_tiles(PASS_BORN, pb, b->grid_pair[PASS_BORN], b->shape[PASS_BORN], st); })) != cudaSuccess)
-      return e;
+    if ((e = tm(kTimBorn, [&] { return enqueue_pass(b, PASS_BORN, pb, st); })) != cudaSuccess) return e;
     if (!fuse_finalize &&
         (e = tm(kTimFinalize, [&] { return launch_born_finalize(fa, st); })) != cudaSuccess)
       return e;
   }
+  pa.early = gb;  // the descreening pass lies between the positions and what follows
   pa.sched = b->sched + 2 * PASS_FORCE;
   if (b->force_blocks == 4 && !b->pl_on) {
     PairArgs p4 = pa;
@@ -1064,9 +1091,7 @@ static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_ene
     p4.n_items = b->n_items4;
     p4.item_count = b->item_count4;
     if ((e = tm(kTimForce, [&] { return launch_force4(p4, b->grid4, b->shape4, st); })) != cudaSuccess) return e;
-  } else if ((e = tm(kTimForce, [&] {
-                return launch_tiles(PASS_FORCE, pa, b->grid_pair[PASS_FORCE], b->shape[PASS_FORCE], st);
-              })) != cudaSuccess) {
+  } else if ((e = tm(kTimForce, [&] { return enqueue_pass(b, PASS_FORCE, pa, st); })) != cudaSuccess) {
     return e;
   }
   pa.sched = b->sched + 2 * PASS_CHAIN;
@@ -1081,8 +1106,7 @@ static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_ene
     pa.n_bonded_chunks = (n_bonded + kBondedChunk - 1) / kBondedChunk;
   }
   if (gb)
-    if ((e = tm(kTimChain, [&] { return launch_tiles(PASS_CHAIN, pa, b->grid_pair[PASS_CHAIN], b->shape[PASS_CHAIN], st); })) != cudaSuccess)
-      return e;
+    if ((e = tm(kTimChain, [&] { return enqueue_pass(b, PASS_CHAIN, pa, st); })) != cudaSuccess) return e;
   if (fuse_bonded) return cudaSuccess;
   return tm(kTimBonded, [&] { return launch_bonded(ba, b->grid_bonded, st); });
 }

@@ -130,6 +130,8 @@ struct pb2_batch {
   int shape[3] = {0, 0, 0};  // block shape of each pair pass (index into the compiled shapes)
   int fuse = PB2_FUSE_BONDED;  // PB2_FUSE_* bits: work folded into the pair passes
   int grid_bonded = 1;
+  int team = 0;                  // warps per tile of the pair passes (0: one, tile2_kernel)
+  int grid_team[3] = {1, 1, 1};
   cudaStream_t cap_stream = nullptr;
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
   bool profiling = false;

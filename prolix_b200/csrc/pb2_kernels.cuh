@@ -75,6 +75,7 @@ struct PairArgs {
   long long *energy;
   int32_t cut;              // any cutoff active
   int32_t *sched;           // (next item, finished warps) of this pass; zero between launches
+  int32_t early;            // 1: the positions and boxes are older than the launch before this one
   // pair list (cutoff runs; NULL otherwise): items come from pl_items[pl_ctl[1]],
   // pl_ctl[2 + pl_ctl[1]] of them, and an item's tiles t in [jb0, jb1) are
   // the j-blocks pl_jlist[t]
@@ -244,6 +245,10 @@ cudaError_t launch_lbfgs(int op, const LbfgsArgs &a, int last_trial, cudaStream_
 constexpr int kShapesPerPass = 3;
 int tile_shape(int pass, int shape, int *threads, int *min_blocks);
 cudaError_t launch_tiles(int pass, const PairArgs &a, int grid, int shape, cudaStream_t st);
+// A pair pass with one thread block (8 or 4 warps) per tile; the same
+// sums as launch_tiles bit for bit.
+cudaError_t launch_team(int pass, int warps, const PairArgs &a, int grid, cudaStream_t st);
+int team_occupancy(int pass, int warps, bool cut);
 // The descreening (pass 0) and energy (pass 1) kernels, and between them the
 // FP64 Born radii with the per-atom energies.
 cudaError_t launch_energy64(int pass, const Energy64Args &a, int grid, cudaStream_t st);

@@ -172,15 +172,20 @@ __device__ __forceinline__ void rotate_force_rest(Acc &tj, int src, const TileCo
   if (K.use_gb) tj.a3 = shfl_next(tj.a3, src);
 }
 
-__device__ __forceinline__ void load_pdata(const PairArgs &a, int g, int pass, bool use_gb, float ro_max,
-                                           PData &P) {
-  const float4 p = a.posq[g], c = a.par[g];
-  P.x = p.x; P.y = p.y; P.z = p.z; P.q = p.w;
+__device__ __forceinline__ void load_par(const PairArgs &a, int g, float ro_max, PData &P) {
+  const float4 c = a.par[g];
   P.hs = c.x; P.se = c.y; P.ro = c.z; P.sr = c.w;
   const float t = fmaxf(P.sr * 2.5f, P.sr + ro_max);  // 2.5 = 1 / sqrt(kSeriesUNear)
   P.t2 = t * t;
   P.s2 = P.sr * P.sr;
   P.s3 = P.s2 * P.sr;
+}
+__device__ __forceinline__ void load_pos(const PairArgs &a, int g, PData &P) {
+  const float4 p = a.posq[g];
+  P.x = p.x; P.y = p.y; P.z = p.z; P.q = p.w;
+}
+// The Born data (after load_par).
+__device__ __forceinline__ void load_born(const PairArgs &a, int g, int pass, bool use_gb, PData &P) {
   P.B = P.iB = P.dedi = P.rB = 0.f;
   if ((pass == PASS_FORCE && use_gb) || pass == PASS_CHAIN) {
     const float4 b = a.born[g];
@@ -192,6 +197,12 @@ __device__ __forceinline__ void load_pdata(const PairArgs &a, int g, int pass, b
     P.se *= kSqrtHalf;
     P.B *= 2.f;
   }
+}
+__device__ __forceinline__ void load_pdata(const PairArgs &a, int g, int pass, bool use_gb, float ro_max,
+                                           PData &P) {
+  load_pos(a, g, P);
+  load_par(a, g, ro_max, P);
+  load_born(a, g, pass, use_gb, P);
 }
 
 // ---------------------------------------------------------------- force pass
@@ -244,21 +255,22 @@ struct Acc2F {
 struct ForceMasks {
   uint32_t R0, R1, X0, X1, Q0, Q1;
 };
+// The masks as step k0 finds them.
 __device__ __forceinline__ ForceMasks force_masks(uint32_t V0, uint32_t V1, uint32_t E0, uint32_t E1, uint32_t S0,
-                                                  uint32_t S1) {
-  return ForceMasks{__brev(V0), __brev(V1), __brev(E0), __brev(E1), __brev(S0), __brev(S1)};
+                                                  uint32_t S1, int k0 = 0) {
+  return ForceMasks{__brev(V0) << k0, __brev(V1) << k0, __brev(E0) << k0,
+                    __brev(E1) << k0, __brev(S0) << k0, __brev(S1) << k0};
 }
 
-// One step of one packed pair of i-blocks against the j atom J: the i-side
-// sums into ti, the j-side sums into tj (not rotated here).  Both the
-// two-block and the four-block force kernels step through this function,
-// so their sums are the same bit for bit.
+// One step of one packed pair of i-blocks against the j atom J: the factors
+// (force_pair_factors: g, the force over the distance vector, and h, the
+// numerator of dE/dB), then the i-side sums into ti and the j-side sums into
+// tj (not rotated here).  Every force kernel uses these functions, so their
+// sums are the same bit for bit.
 template <bool CUT, bool FULL, bool EXCL>
-__device__ __forceinline__ void force_pair_step(const FData2 &I, const JF2 &J, Acc2F &ti, Acc &tj, ForceMasks &M,
-                                                const TileConst &K) {
-  const float2 dx = __fadd2_rn(I.x, J.mx);
-  const float2 dy = __fadd2_rn(I.y, J.my);
-  const float2 dz = __fadd2_rn(I.z, J.mz);
+__device__ __forceinline__ void force_pair_factors(const FData2 &I, const JF2 &J, float2 dx, float2 dy, float2 dz,
+                                                   ForceMasks &M, const TileConst &K, float2 &g_out,
+                                                   float2 &h_out) {
   float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
   if (!FULL) {
     r2 = make_float2((int32_t)M.R0 < 0 ? r2.x : kFarR2, (int32_t)M.R1 < 0 ? r2.y : kFarR2);
@@ -266,6 +278,7 @@ __device__ __forceinline__ void force_pair_step(const FData2 &I, const JF2 &J, A
     M.R1 <<= 1;
   }
   float2 g = make_float2(0.f, 0.f);
+  h_out = make_float2(0.f, 0.f);
   if (K.use_gb) {
     // E = P qq / f, f^2 = r^2 + B_i B_j e^(-r^2 / 4 B_i B_j); with
     // A2 = 2 P qq / f^3:  -dE/dr / r = A2 (1 - e / 4), and
@@ -286,9 +299,7 @@ __device__ __forceinline__ void force_pair_step(const FData2 &I, const JF2 &J, A
     if (CUT && K.gcut2 != 0.f) A2 = __fmul2_rn(A2, sel2(r2.x < K.gcut2, r2.y < K.gcut2, 1.f, 0.f));
     const float2 A2e = __fmul2_rn(A2, ex);
     g = make_float2(__fsub_rn(A2.x, A2e.x), __fsub_rn(A2.y, A2e.y));
-    const float2 h = __fmul2_rn(A2e, __fadd2_rn(bb, r2));
-    ti.a3 = __fadd2_rn(ti.a3, h);
-    tj.a3 = tj.a3 + h.x + h.y;
+    h_out = __fmul2_rn(A2e, __fadd2_rn(bb, r2));
   }
   if (K.use_lj || K.use_coul) {
     const float2 inv_r = rsqrt2(r2);
@@ -317,6 +328,21 @@ __device__ __forceinline__ void force_pair_step(const FData2 &I, const JF2 &J, A
     }
     if (CUT && K.cut2 != 0.f) s = __fmul2_rn(s, sel2(r2.x < K.cut2, r2.y < K.cut2, 1.f, 0.f));
     g = __ffma2_rn(s, inv_r2, g);
+  }
+  g_out = g;
+}
+
+template <bool CUT, bool FULL, bool EXCL>
+__device__ __forceinline__ void force_pair_step(const FData2 &I, const JF2 &J, Acc2F &ti, Acc &tj, ForceMasks &M,
+                                                const TileConst &K) {
+  const float2 dx = __fadd2_rn(I.x, J.mx);
+  const float2 dy = __fadd2_rn(I.y, J.my);
+  const float2 dz = __fadd2_rn(I.z, J.mz);
+  float2 g, h;
+  force_pair_factors<CUT, FULL, EXCL>(I, J, dx, dy, dz, M, K, g, h);
+  if (K.use_gb) {
+    ti.a3 = __fadd2_rn(ti.a3, h);
+    tj.a3 = tj.a3 + h.x + h.y;
   }
   ti.a0 = __ffma2_rn(g, dx, ti.a0);
   ti.a1 = __ffma2_rn(g, dy, ti.a1);
@@ -519,6 +545,35 @@ __device__ __forceinline__ void cf_drain(CfQueue &Q, int lane) {
   Q.n = 0;
 }
 
+// The near-tile test of a step's two pairs: those outside the series' domain
+// go to the warp's queue (CAP entries) with their series terms zeroed.  All
+// lanes of the warp arrive here.  jg: the j atom the lane meets at this step.
+template <int PASS, int CAP>
+__device__ __forceinline__ void cf_push(const PData2 &I, const JD2 &J, BCPair2 &P, int jg, const TileConst &K,
+                                        CfQueue &Q) {
+  // r >= t_i and r >= t_j give (s/r)^2 <= kSeriesUNear for both radii and
+  // r - s >= rho~_max >= rho~ for both directions: a sufficient test in two
+  // instructions (it sends about 1.3 % of near-tile pairs of compact
+  // chains to the closed form, barely more than the exact test)
+  const bool n0 = P.ok0 && !(P.r2.x >= fmaxf(I.t2.x, J.t2));
+  const bool n1 = P.ok1 && !(P.r2.y >= fmaxf(I.t2.y, J.t2));
+  const unsigned b0 = __ballot_sync(kFull, n0), b1 = __ballot_sync(kFull, n1);
+  if (b0 | b1) {  // warp-uniform
+    const int c0 = __popc(b0), cnt = c0 + __popc(b1);
+    if (Q.n + cnt > CAP) cf_drain<PASS>(Q, K.lane);
+    const unsigned lt = (1u << K.lane) - 1u;
+    if (n0) {
+      Q.q[Q.n + __popc(b0 & lt)] = make_int2(Q.ig0, jg);
+      P.vij.x = 0.f; P.vji.x = 0.f; P.f.x = 0.f;
+    }
+    if (n1) {
+      Q.q[Q.n + c0 + __popc(b1 & lt)] = make_int2(Q.ig1, jg);
+      P.vij.y = 0.f; P.vji.y = 0.f; P.f.y = 0.f;
+    }
+    Q.n += cnt;
+  }
+}
+
 // FAR: both tiles lie in the series' domain (no per-pair test); otherwise
 // each pair is tested, and those outside the domain go to the warp's
 // closed-form queue with their series terms zeroed.
@@ -537,30 +592,7 @@ __device__ __forceinline__ void run_bc_tile2(const PData2 &I, const JTile &jt, A
       R0 <<= 1;
       R1 <<= 1;
     }
-    if (!FAR) {
-      // r >= t_i and r >= t_j give (s/r)^2 <= kSeriesUNear for both radii and
-      // r - s >= rho~_max >= rho~ for both directions: a sufficient test in two
-      // instructions (it sends about 1.3 % of near-tile pairs of compact
-      // chains to the closed form, barely more than the exact test)
-      const bool n0 = P.ok0 && !(P.r2.x >= fmaxf(I.t2.x, J.t2));
-      const bool n1 = P.ok1 && !(P.r2.y >= fmaxf(I.t2.y, J.t2));
-      const unsigned b0 = __ballot_sync(kFull, n0), b1 = __ballot_sync(kFull, n1);
-      if (b0 | b1) {  // warp-uniform
-        const int c0 = __popc(b0), cnt = c0 + __popc(b1);
-        if (Q.n + cnt > kCfCap) cf_drain<PASS>(Q, K.lane);
-        const unsigned lt = (1u << K.lane) - 1u;
-        const int jg = Q.jg0 + ((K.lane + k) & 31);  // the j atom this lane holds at step k
-        if (n0) {
-          Q.q[Q.n + __popc(b0 & lt)] = make_int2(Q.ig0, jg);
-          P.vij.x = 0.f; P.vji.x = 0.f; P.f.x = 0.f;
-        }
-        if (n1) {
-          Q.q[Q.n + c0 + __popc(b1 & lt)] = make_int2(Q.ig1, jg);
-          P.vij.y = 0.f; P.vji.y = 0.f; P.f.y = 0.f;
-        }
-        Q.n += cnt;
-      }
-    }
+    if (!FAR) cf_push<PASS, kCfCap>(I, J, P, Q.jg0 + ((K.lane + k) & 31), K, Q);
     bc_accumulate2<PASS>(I, J, P, ti, tj);
     tj.a0 = shfl_next(tj.a0, src);
     if (PASS == PASS_CHAIN) {
@@ -897,6 +929,313 @@ __global__ void __launch_bounds__(THREADS, MINB)
   }
 }
 
+// --------------------------------------------------------------------- teams
+//
+// What a batch of few tiles waits for is one warp's 32 steps: at N = 166 a
+// pass is 12 tiles on 148 SMs, and each step's sums wait for the step before.
+// A team, the W warps of a thread block, shares a tile instead: each warp
+// evaluates 32 / W steps' factors (independent of one another) into shared
+// memory, and then the sums of the i and j sides, component by component,
+// are taken by different warps, each in the order of the steps.  The factors
+// and the order of the additions are those of tile2_kernel, so the sums are
+// the same bit for bit, and a batch may use either kernel.  (Parts of a tile
+// summed on their own were as fast for one small system, but rounded
+// differently, and kept so in large batches they cost those 5 to 10 %.)
+// us per step with one warp per tile and with teams: 166 atoms 34.2, 20.9;
+// 896 atoms 36.9, 22.5.
+
+// A tile in shared memory.  Entry k * 32 + l of the factors is lane l's at
+// step k: (g, h) of the force pass in g4; (vij, vji) of the descreening pass
+// in g4 and f in g2; the chain rule's force over the distance vector in g2.
+template <int PASS>
+struct TeamShared {
+  JTile jt;
+  float2 ix[3][32];                            // the i atoms' packed positions
+  float2 rb[32];                               // their 1 / B
+  float jrb[32];
+  float4 g4[PASS == PASS_CHAIN ? 1 : 1024];
+  float2 g2[PASS == PASS_FORCE ? 1 : 1024];
+  int next;
+};
+constexpr int kTeamQueue = 128;  // queued closed-form pairs per warp
+
+// Steps k0 .. k0 + KN - 1 of the descreening and chain passes: the factors
+// that bc_accumulate2 sums.  FAR and the queue as in run_bc_tile2.
+template <int PASS, bool FAR, bool CUT, int TIER, int KN>
+__device__ __forceinline__ void team_bc_steps(const PData2 &I, TeamShared<PASS> &T, uint32_t V0, uint32_t V1, int k0,
+                                              const TileConst &K, CfQueue &Q) {
+  uint32_t R0 = __brev(V0) << k0, R1 = __brev(V1) << k0;
+#pragma unroll(KN < 8 ? KN : 4)
+  for (int k = 0; k < KN; ++k) {
+    const int e = K.lane + k0 + k;
+    const JD2 J = load_jd<PASS, FAR>(T.jt, e);
+    BCPair2 P;
+    bc_series2<PASS, CUT, false, TIER>(I, J, (int32_t)R0 < 0, (int32_t)R1 < 0, P, K);
+    R0 <<= 1;
+    R1 <<= 1;
+    if (!FAR) cf_push<PASS, kTeamQueue>(I, J, P, Q.jg0 + (e & 31), K, Q);
+    const int o = (k0 + k) * 32 + K.lane;
+    if constexpr (PASS == PASS_BORN) {
+      T.g4[o] = make_float4(P.vij.x, P.vij.y, P.vji.x, P.vji.y);
+      T.g2[o] = P.f;
+    } else {
+      T.g2[o] = __fmul2_rn(__ffma2_rn(I.dedi, P.vij, __fmul2_rn(J.dedi, P.vji)), P.f);
+    }
+  }
+}
+
+// One component of the force on a tile's atoms, in the order of the steps:
+// g the factor, x the packed i coordinates, mx minus the j coordinate.
+// i side (lane: i atom of each block), then j side (lane: j atom).
+template <int PASS>
+__device__ __forceinline__ float2 team_factor(const TeamShared<PASS> &T, int o) {
+  if constexpr (PASS == PASS_FORCE) {
+    const float4 v = T.g4[o];
+    return make_float2(v.x, v.y);
+  } else {
+    return T.g2[o];
+  }
+}
+__device__ __forceinline__ float2 jt_minus(const JTile &t, int c, int e) {  // (-x, -x) of component c
+  const float4 v = t[c >> 1][e];
+  return c & 1 ? hi2(v) : lo2(v);
+}
+template <int PASS>
+__device__ __forceinline__ float2 team_i_sum(const TeamShared<PASS> &T, int c, int lane) {
+  const float2 x = T.ix[c][lane];
+  float2 t = make_float2(0.f, 0.f);
+#pragma unroll 8
+  for (int k = 0; k < 32; ++k)
+    t = __ffma2_rn(team_factor<PASS>(T, k * 32 + lane), __fadd2_rn(x, jt_minus(T.jt, c, lane + k)), t);
+  return t;
+}
+template <int PASS>
+__device__ __forceinline__ float team_j_sum(const TeamShared<PASS> &T, int c, int lane) {
+  const float2 mx = jt_minus(T.jt, c, lane);
+  float t = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < 32; ++k) {
+    const int l = (lane - k) & 31;
+    const float2 g = team_factor<PASS>(T, k * 32 + l), d = __fadd2_rn(T.ix[c][l], mx);
+    t = fmaf(-g.x, d.x, fmaf(-g.y, d.y, t));
+  }
+  return t;
+}
+
+template <int PASS, bool CUT, bool ALL, int W>
+__global__ void __launch_bounds__(32 * W) team_kernel(const __grid_constant__ PairArgs a) {
+  constexpr int KN = 32 / W;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  TileConst K;
+  K.use_gb = ALL || (a.terms & PB2_USE_GB) != 0;
+  K.use_lj = ALL || (a.terms & PB2_USE_LJ) != 0;
+  K.use_coul = ALL || (a.terms & PB2_USE_COULOMB) != 0;
+  K.src = (lane + 1) & 31;
+  K.lane = lane;
+  __shared__ TeamShared<PASS> T;
+  __shared__ int2 s_cfq[PASS == PASS_FORCE ? 1 : W][PASS == PASS_FORCE ? 1 : kTeamQueue];
+  const float bscale = PASS == PASS_BORN ? (float)kBornScale : (float)kForceScale;
+  CfQueue Q;
+  Q.c = {a.posq, a.par, a.born, a.dedb_acc, a.born_acc, a.fx, a.fy, a.fz};
+  Q.q = s_cfq[PASS == PASS_FORCE ? 0 : w];
+  Q.n = 0;
+  Q.bscale = bscale;
+  const uint32_t diag_mask = lane == 31 ? 0u : (0xffffffffu << (lane + 1));
+
+  // The launch before is waited for only where its results are first read:
+  // first the bonded chunks (they read positions, and add to accumulators)
+  // and what no kernel of a step writes, then the positions and boxes (older
+  // than the launch before when a.early), then the Born data.
+  bool waited = false;
+  auto wait = [&] {
+    if (!waited) {
+      pdl_wait();
+      pdl_trigger();
+      waited = true;
+    }
+  };
+  const bool plm = CUT && a.pl_ctl != nullptr;
+  const TileItem *items = a.items;
+  int n_items = 0;
+  if (plm) {  // written by the list's update: with the descreening pass between, older than the launch before
+    if (!a.early) wait();
+    const int cur = a.pl_ctl[PL_CUR];
+    items = cur ? a.pl_items1 : a.pl_items0;
+    n_items = a.pl_ctl[PL_COUNT0 + cur];
+  } else {
+    n_items = *a.item_count;
+  }
+  // units: W bonded chunks each (the longest), then the items
+  const int n_bonded = PASS == PASS_CHAIN ? (a.n_bonded_chunks + W - 1) / W : 0;
+  for (int u = (int)blockIdx.x; u < n_bonded + n_items;) {
+    if (u < n_bonded) {
+      const int t = (u * W + w) * kBondedChunk + lane;
+      if (t < bonded_total(a.bonded)) bonded_term_call(a.bonded, t);
+    } else {
+      const TileItem item = items[u - n_bonded];
+      const SysInfo &S = a.sys[item.sys];
+      const int n = S.n, off = S.off;
+      K.cut2 = S.cutoff2; K.gcut2 = S.gb_cutoff2; K.bcut2 = S.born_cut2;
+      K.pref = S.pref; K.kcoul = S.kcoul; K.lj14 = S.lj14; K.coul14 = S.coul14;
+      const int ib0 = item.iblk, ib1 = ib0 + 1;
+      const bool has1 = ib1 < S.nblk;
+      const int gib0 = S.blk_base + ib0, gib1 = S.blk_base + (has1 ? ib1 : ib0);
+      const int il0 = ib0 * 32 + lane, il1 = ib1 * 32 + lane;
+      const bool iv0 = il0 < n, iv1 = il1 < n;  // il1 >= n whenever !has1
+      const int ig0 = off + (iv0 ? il0 : n - 1), ig1 = off + (iv1 ? il1 : n - 1);
+      int2 ent = make_int2(-1, -1);
+      if (PASS == PASS_FORCE) {
+        if (lane < kExclPerBlock) ent = a.excl_ent[gib0 * kExclPerBlock + lane];
+        else if (has1) ent = a.excl_ent[gib1 * kExclPerBlock + lane - kExclPerBlock];
+      }
+      PData I0, I1;
+      load_par(a, ig0, S.ro_max, I0);
+      load_par(a, ig1, S.ro_max, I1);
+      for (int tt = item.jb0; tt < item.jb1; ++tt) {
+        const int jb = plm ? a.pl_jlist[tt] : tt;
+        const int jl0 = jb * 32, jl = jl0 + lane;
+        const bool jvalid = jl < n;
+        const int jg = off + (jvalid ? jl : n - 1);
+        PData J;
+        load_par(a, jg, S.ro_max, J);
+        uint32_t E0 = 0u, S0 = 0u, E1 = 0u, S1 = 0u;
+        if constexpr (PASS == PASS_FORCE) {
+          const unsigned hit = __ballot_sync(kFull, ent.x == jb);
+          const unsigned hit0 = hit & 0xffffu, hit1 = hit & 0xffff0000u;
+          if (hit0) {
+            const ExclRow r = a.excl_rows[__shfl_sync(kFull, ent.y, __ffs(hit0) - 1) + lane];
+            E0 = rotr32(r.excl, lane); S0 = rotr32(r.s14, lane);
+          }
+          if (hit1) {
+            const ExclRow r = a.excl_rows[__shfl_sync(kFull, ent.y, __ffs(hit1) - 1) + lane];
+            E1 = rotr32(r.excl, lane); S1 = rotr32(r.s14, lane);
+          }
+        }
+        if (!a.early) wait();
+        load_pos(a, ig0, I0);
+        load_pos(a, ig1, I1);
+        load_pos(a, jg, J);
+        float d2 = 0.f;
+        if (CUT || PASS != PASS_FORCE) {
+          d2 = box_dist2(a.bbox, gib0, S.blk_base + jb);
+          if (has1 && jb > ib0) d2 = fminf(d2, box_dist2(a.bbox, gib1, S.blk_base + jb));
+        }
+        wait();
+        if (CUT) {
+          float reach2 = K.bcut2;
+          if (PASS == PASS_FORCE) reach2 = (K.gcut2 == 0.f || K.cut2 == 0.f) ? 0.f : fmaxf(K.gcut2, K.cut2);
+          if (reach2 > 0.f && d2 >= reach2) continue;  // no pair within reach (block-uniform)
+        }
+        load_born(a, ig0, PASS, K.use_gb, I0);
+        load_born(a, ig1, PASS, K.use_gb, I1);
+        load_born(a, jg, PASS, K.use_gb, J);
+        if (w == 0) {
+          store_j<PASS>(T.jt, lane, J);
+          T.jrb[lane] = J.rB;
+        }
+        if (w == W - 1) {
+          T.ix[0][lane] = make_float2(I0.x, I1.x);
+          T.ix[1][lane] = make_float2(I0.y, I1.y);
+          T.ix[2][lane] = make_float2(I0.z, I1.z);
+          T.rb[lane] = make_float2(I0.rB, I1.rB);
+        }
+        // pair validity of lane i with j-lane c: both exist, j > i on a diagonal
+        const int nj = n - jl0;
+        const uint32_t jmask = nj >= 32 ? 0xffffffffu : ((1u << nj) - 1u);
+        uint32_t C0 = iv0 ? jmask : 0u, C1 = iv1 ? jmask : 0u;
+        if (jb == ib0) {
+          C0 &= diag_mask;
+          C1 = 0u;
+        } else if (jb == ib1) {
+          C1 &= diag_mask;
+        }
+        const uint32_t V0 = rotr32(C0, lane), V1 = rotr32(C1, lane);
+        const int k0 = w * KN;
+        __syncthreads();
+        if constexpr (PASS == PASS_FORCE) {
+          const FData2 IF = {make_float2(I0.x, I1.x), make_float2(I0.y, I1.y), make_float2(I0.z, I1.z),
+                             make_float2(I0.hs, I1.hs), make_float2(I0.se, I1.se),
+                             make_float2(I0.B, I1.B), make_float2(I0.iB, I1.iB),
+                             make_float2(2.f * K.pref * I0.q, 2.f * K.pref * I1.q),
+                             make_float2(K.kcoul * I0.q, K.kcoul * I1.q)};
+          ForceMasks M = force_masks(V0, V1, E0, E1, S0, S1, k0);
+#pragma unroll(KN < 8 ? KN : 4)
+          for (int k = 0; k < KN; ++k) {
+            const JF2 Jk = load_jf(T.jt, lane + k0 + k);
+            float2 g, h;
+            force_pair_factors<CUT, false, true>(IF, Jk, __fadd2_rn(IF.x, Jk.mx), __fadd2_rn(IF.y, Jk.my),
+                                                 __fadd2_rn(IF.z, Jk.mz), M, K, g, h);
+            T.g4[(k0 + k) * 32 + lane] = make_float4(g.x, g.y, h.x, h.y);
+          }
+        } else {
+          const PData2 I2 = pack2(I0, I1);
+          const float *tier2 = S.tier2[PASS == PASS_BORN ? 0 : 1];
+          Q.ig0 = ig0; Q.ig1 = ig1; Q.jg0 = off + jl0;
+          if (d2 >= tier2[0]) team_bc_steps<PASS, true, CUT, 0, KN>(I2, T, V0, V1, k0, K, Q);
+          else if (d2 >= tier2[1]) team_bc_steps<PASS, true, CUT, 1, KN>(I2, T, V0, V1, k0, K, Q);
+          else if (d2 >= tier2[2]) team_bc_steps<PASS, true, CUT, 2, KN>(I2, T, V0, V1, k0, K, Q);
+          else if (d2 >= S.far2) team_bc_steps<PASS, true, CUT, 3, KN>(I2, T, V0, V1, k0, K, Q);
+          else team_bc_steps<PASS, false, CUT, 3, KN>(I2, T, V0, V1, k0, K, Q);
+        }
+        __syncthreads();
+        // the sums, one per task: the i side's x, y, z (and dE/dB), the j side's
+        constexpr int kSide = PASS == PASS_BORN ? 1 : PASS == PASS_FORCE ? 4 : 3;
+#pragma unroll 1
+        for (int task = w; task < 2 * kSide; task += W) {
+          const int c = task < kSide ? task : task - kSide;
+          const bool iside = task < kSide;
+          long long *acc = PASS == PASS_BORN ? a.born_acc : c == 0 ? a.fx : c == 1 ? a.fy : c == 2 ? a.fz : a.dedb_acc;
+          if (PASS == PASS_FORCE && c == 3 && !K.use_gb) continue;
+          float2 s = make_float2(0.f, 0.f);  // i side: both atoms'; j side: .x
+          if constexpr (PASS == PASS_BORN) {
+#pragma unroll 8
+            for (int k = 0; k < 32; ++k) {
+              const int o = k * 32 + (iside ? lane : (lane - k) & 31);
+              const float4 v = T.g4[o];
+              const float2 f = T.g2[o];
+              if (iside) s = __ffma2_rn(make_float2(v.x, v.y), f, s);
+              else s.x = fmaf(v.z, f.x, fmaf(v.w, f.y, s.x));
+            }
+          } else if (c == 3) {
+            if constexpr (PASS == PASS_FORCE) {
+#pragma unroll 8
+              for (int k = 0; k < 32; ++k) {
+                const float4 v = T.g4[k * 32 + (iside ? lane : (lane - k) & 31)];
+                if (iside) s = __fadd2_rn(s, make_float2(v.z, v.w));
+                else s.x = s.x + v.z + v.w;
+              }
+            }
+            const float2 rb = T.rb[lane];
+            if (iside) s = make_float2(s.x * (-0.5f * rb.x), s.y * (-0.5f * rb.y));
+            else s.x = s.x * (-0.5f * T.jrb[lane]);
+          } else if (iside) {
+            s = team_i_sum<PASS>(T, c, lane);
+          } else {
+            s.x = team_j_sum<PASS>(T, c, lane);
+          }
+          if (iside) {
+            if (iv0) atomic_add_fix(&acc[ig0], to_fix_f(s.x, bscale));
+            if (iv1) atomic_add_fix(&acc[ig1], to_fix_f(s.y, bscale));
+          } else if (jvalid) {
+            atomic_add_fix(&acc[jg], to_fix_f(s.x, bscale));
+          }
+        }
+        if (PASS != PASS_FORCE && Q.n > 0) cf_drain<PASS>(Q, lane);
+        __syncthreads();  // the tile's shared data are read before the next tile's are written
+      }
+    }
+    if (threadIdx.x == 0) T.next = (int)gridDim.x + atomicAdd(&a.sched[0], 1);
+    __syncthreads();
+    u = T.next;
+    __syncthreads();
+  }
+  if (!waited) pdl_wait();
+  if (threadIdx.x == 0 && atomicAdd(&a.sched[1], 1) == (int)gridDim.x - 1) {
+    a.sched[0] = 0;
+    a.sched[1] = 0;
+  }
+}
+
 // The force pass with four i-blocks per warp: work items (system, i-block
 // ib with ib % 4 == 0, j-blocks [jb0, jb1)); lane l owns atom l of blocks
 // ib .. ib + 3, in two packed pairs (ib, ib + 1) and (ib + 2, ib + 3) that
@@ -1166,6 +1505,45 @@ cudaError_t launch_tiles(int pass, const PairArgs &a, int grid, int shape, cudaS
     }
   }
   return cudaGetLastError();
+}
+
+template <int PASS, bool CUT, bool ALL, int W>
+static cudaError_t team_do(const PairArgs *a, int grid, cudaStream_t st, int *occ) {
+  if (!occ) return launch_after(team_kernel<PASS, CUT, ALL, W>, grid, 32 * W, st, *a);
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, team_kernel<PASS, CUT, ALL, W>, 32 * W, 0);
+}
+template <int PASS, bool CUT, bool ALL>
+static cudaError_t team_w(int warps, const PairArgs *a, int grid, cudaStream_t st, int *occ) {
+  if (warps == 8) return team_do<PASS, CUT, ALL, 8>(a, grid, st, occ);
+  return team_do<PASS, CUT, ALL, 4>(a, grid, st, occ);
+}
+static cudaError_t team_any(int pass, int warps, bool cut, bool all, const PairArgs *a, int grid, cudaStream_t st,
+                            int *occ) {
+  if (pass == PASS_BORN)
+    return cut ? team_w<PASS_BORN, true, false>(warps, a, grid, st, occ)
+               : team_w<PASS_BORN, false, false>(warps, a, grid, st, occ);
+  if (pass == PASS_CHAIN)
+    return cut ? team_w<PASS_CHAIN, true, false>(warps, a, grid, st, occ)
+               : team_w<PASS_CHAIN, false, false>(warps, a, grid, st, occ);
+  if (cut)
+    return all ? team_w<PASS_FORCE, true, true>(warps, a, grid, st, occ)
+               : team_w<PASS_FORCE, true, false>(warps, a, grid, st, occ);
+  return all ? team_w<PASS_FORCE, false, true>(warps, a, grid, st, occ)
+             : team_w<PASS_FORCE, false, false>(warps, a, grid, st, occ);
+}
+cudaError_t launch_team(int pass, int warps, const PairArgs &a, int grid, cudaStream_t st) {
+  if (grid <= 0) return cudaSuccess;
+  const uint32_t t = PB2_USE_GB | PB2_USE_LJ | PB2_USE_COULOMB;
+  return team_any(pass, warps, a.cut != 0, (a.terms & t) == t, &a, grid, st, nullptr);
+}
+int team_occupancy(int pass, int warps, bool cut) {
+  int m = 1 << 20;
+  for (int all = 0; all < 2; ++all) {
+    int blocks = 0;
+    team_any(pass, warps, cut, all != 0, nullptr, 0, nullptr, &blocks);
+    m = std::min(m, blocks);
+  }
+  return std::max(m, 1);
 }
 
 cudaError_t launch_bbox(const SysInfo *sys, const int32_t *blk_sys, const float4 *posq, float4 *bbox,
