@@ -1528,6 +1528,17 @@ static MinArgs min_args(pb2_batch *b) {
   a.par = b->m_par;
   a.n_total = b->n_total;
   a.n_sys = b->n_sys;
+  a.chunks = b->m_chunks;
+  a.chunk0 = b->m_chunk0;
+  a.n_chunks = b->m_n_chunks;
+  a.part = b->m_part;
+  a.sys_done = b->m_done;
+  a.mix_f = b->m_sys + 4 * (size_t)b->n_sys;
+  a.mix_p = b->m_sys + 5 * (size_t)b->n_sys;
+  a.sys_flags = b->m_flags;
+  a.bbox = b->bbox;
+  a.pl_ref = b->pl_on ? b->pl_ref : nullptr;
+  a.pl_ctl = b->pl_on ? b->pl_ctl : nullptr;
   return a;
 }
 
@@ -1543,9 +1554,27 @@ extern "C" int pb2_min_setup(pb2_batch *b, const uint8_t *heavy, const uint8_t *
     b->m_xb = D.alloc<double>(3 * N);
     b->m_best = D.alloc<double>(3 * N);
     b->m_par = D.alloc<double>(kMinNPar);
-    b->m_sys = D.alloc<double>(4 * (size_t)b->n_sys);
+    b->m_sys = D.alloc<double>(6 * (size_t)b->n_sys);
     b->m_npos = D.alloc<int32_t>(b->n_sys);
     b->m_sel = D.alloc<uint8_t>(N);
+    std::vector<int2> chunks;
+    std::vector<int32_t> first;
+    for (int s = 0; s < b->n_sys; ++s) {
+      first.push_back((int)chunks.size());
+      for (int k = 0; k < b->sys_host[s].nblk; k += kMinChunkBlocks) chunks.push_back(make_int2(s, k));
+    }
+    first.push_back((int)chunks.size());
+    b->m_n_chunks = (int)chunks.size();
+    b->m_chunks = D.alloc<int2>(chunks.size());
+    b->m_chunk0 = D.alloc<int32_t>(first.size());
+    b->m_part = D.alloc<double>(3 * chunks.size());
+    b->m_done = D.alloc<int32_t>(b->n_sys);
+    b->m_flags = D.alloc<int32_t>(b->n_sys);
+    if (!b->m_chunks || !b->m_chunk0 || !b->m_part || !b->m_done || !b->m_flags)
+      return fail(ctx, PB2_ENOMEM, "minimiser allocation failed");
+    int rc;
+    if ((rc = upload(ctx, b->m_chunks, chunks)) || (rc = upload(ctx, b->m_chunk0, first))) return rc;
+    CUDA_TRY(ctx, cudaMemset(b->m_done, 0, b->n_sys * sizeof(int32_t)));
     if (!b->m_x0 || !b->m_ft || !b->m_xb || !b->m_best || !b->m_par || !b->m_sys || !b->m_npos || !b->m_sel)
       return fail(ctx, PB2_ENOMEM, "minimiser allocation failed");
   }
@@ -1584,12 +1613,11 @@ static int min_graph(pb2_batch *b, int mode, int chunk, cudaGraphExec_t *out) {
   for (int t = 0; t < chunk && err == cudaSuccess; ++t) {
     if (mode == 0) {
       err = launch_min(kMinOpSd, ma, nullptr, cs);
-      if (err == cudaSuccess) err = enqueue_forces(b, cs, false);
+      if (err == cudaSuccess) err = enqueue_forces(b, cs, false, true);
     } else {
-      err = launch_min(kMinOpFireBegin, ma, nullptr, cs);
-      if (err == cudaSuccess) err = launch_min(kMinOpFireDrift, ma, nullptr, cs);
-      if (err == cudaSuccess) err = enqueue_forces(b, cs, false);
-      if (err == cudaSuccess) err = launch_min(kMinOpFireMix, ma, nullptr, cs);
+      err = launch_min(kMinOpFireMove, ma, nullptr, cs);
+      if (err == cudaSuccess) err = enqueue_forces(b, cs, false, true);
+      if (err == cudaSuccess) err = launch_min(kMinOpFireClose, ma, nullptr, cs);
     }
   }
   cudaGraph_t g = nullptr;
@@ -1670,6 +1698,7 @@ extern "C" int pb2_min_fire(pb2_batch *b, int32_t n_steps, double k, int32_t kin
   const MinArgs ma = min_args(b);
   CUDA_TRY(b->ctx, launch_min(kMinOpFireInit, ma, nullptr, st));
   if ((rc = min_run(b, 1, n_steps, st))) return rc;
+  CUDA_TRY(b->ctx, launch_min(kMinOpFireEnd, ma, nullptr, st));
   if (flags & PB2_FIRE_KEEP_BEST) CUDA_TRY(b->ctx, launch_min(kMinOpTakeBest, ma, nullptr, st));
   CUDA_TRY(b->ctx, launch_min(kMinOpRollback, ma, nullptr, st));
   b->forces_valid = false;

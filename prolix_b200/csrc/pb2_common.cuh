@@ -103,6 +103,26 @@ __device__ __forceinline__ void atomic_add_fix(long long *addr, long long v) {
   atomicAdd(reinterpret_cast<unsigned long long *>(addr), static_cast<unsigned long long>(v));
 }
 
+// The bounding box of 32-atom block b, whose atom `lane` is at q (lanes past a
+// system's last atom take the block's first).
+__device__ __forceinline__ void block_box(float4 *bbox, int b, int lane, bool valid, float4 q) {
+  const float4 q0 = make_float4(__shfl_sync(kFull, q.x, 0), __shfl_sync(kFull, q.y, 0),
+                                __shfl_sync(kFull, q.z, 0), 0.f);
+  if (!valid) q = q0;
+  float lo[3] = {q.x, q.y, q.z}, hi[3] = {q.x, q.y, q.z};
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = fminf(lo[c], __shfl_xor_sync(kFull, lo[c], o));
+      hi[c] = fmaxf(hi[c], __shfl_xor_sync(kFull, hi[c], o));
+    }
+  if (lane == 0) {
+    bbox[2 * b] = make_float4(lo[0], lo[1], lo[2], 0.f);
+    bbox[2 * b + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
+  }
+}
+
 // Asynchronous global -> shared copies (cp.async): a thread's copies land in
 // groups, in order; cp_async_wait<N>() waits until at most N groups are in
 // flight.  Source and destination aligned to the copy's size.

@@ -48,26 +48,7 @@ __device__ __forceinline__ float4 write_posq(const IntArgs &a, int i, const SysI
 // The step kernels map one warp to one 32-atom block (lane l: atom l of the
 // block), so that the block's bounding box of the new positions -- what the
 // pair kernels cull tiles by -- comes out of the same launch, and so does
-// the pair list's displacement test.  Lanes past a system's last atom take
-// the block's first atom for the box.
-__device__ __forceinline__ void block_box(const IntArgs &a, int b, int lane, bool valid, float4 q) {
-  const float4 q0 = make_float4(__shfl_sync(kFull, q.x, 0), __shfl_sync(kFull, q.y, 0),
-                                __shfl_sync(kFull, q.z, 0), 0.f);
-  if (!valid) q = q0;
-  float lo[3] = {q.x, q.y, q.z}, hi[3] = {q.x, q.y, q.z};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      lo[c] = fminf(lo[c], __shfl_xor_sync(kFull, lo[c], o));
-      hi[c] = fmaxf(hi[c], __shfl_xor_sync(kFull, hi[c], o));
-    }
-  if (lane == 0) {
-    a.bbox[2 * b] = make_float4(lo[0], lo[1], lo[2], 0.f);
-    a.bbox[2 * b + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
-  }
-}
-
+// the pair list's displacement test.
 // The charge and the pair list's reference position, loaded before the
 // step's stores: the FP64 stores could alias the charge and the posq store
 // the reference, and a load ordered after them adds a memory latency at the
@@ -248,7 +229,7 @@ __global__ void __launch_bounds__(32 * kStepWarps, 6) step_kernel(const IntArgs 
         q = step_atom(a, cur.y + lane, s, S, s_in[wl][it & 1], noise, lane);
         moved |= moved_past_half_skin(a, e, S, q);
       }
-      block_box(a, b, lane, valid, q);
+      block_box(a.bbox, b, lane, valid, q);
     }
     __syncwarp();  // the buffer is read before the next block's copies refill it
   }
@@ -387,7 +368,7 @@ __global__ void __launch_bounds__(256, 4) step_guarded_kernel(const IntArgs a) {
       q = step_guarded_atom(a, S.off + l, s, S, e, cap_open);
       moved |= moved_past_half_skin(a, e, S, q);
     }
-    block_box(a, b, lane, valid, q);
+    block_box(a.bbox, b, lane, valid, q);
   }
   if (a.pl_ctl && __any_sync(kFull, moved) && lane == 0) atomicOr(&a.pl_ctl[PL_DIRTY], 1);
 }
@@ -545,7 +526,7 @@ __global__ void __launch_bounds__(128) place_kernel(const IntArgs a, const doubl
       a.fx[i] = 0; a.fy[i] = 0; a.fz[i] = 0;
       moved |= moved_past_half_skin(a, e, S, q);
     }
-    block_box(a, b, lane, valid, q);
+    block_box(a.bbox, b, lane, valid, q);
   }
   if (a.pl_ctl && __any_sync(kFull, moved) && lane == 0) atomicOr(&a.pl_ctl[PL_DIRTY], 1);
 }

@@ -144,7 +144,11 @@ struct pb2_batch {
   Dev mdev;
   bool min_ready = false;
   double *m_x0 = nullptr, *m_ft = nullptr, *m_xb = nullptr, *m_best = nullptr, *m_par = nullptr;
-  double *m_sys = nullptr;  // dt, alpha, best rms, rms: (4, n_sys)
+  double *m_sys = nullptr;  // dt, alpha, best rms, rms, mix_f, mix_p: (6, n_sys)
+  int2 *m_chunks = nullptr;
+  int32_t *m_chunk0 = nullptr, *m_done = nullptr, *m_flags = nullptr;
+  int m_n_chunks = 0;
+  double *m_part = nullptr;
   int32_t *m_npos = nullptr;
   uint8_t *m_sel = nullptr;
   std::map<std::pair<int, int>, cudaGraphExec_t> min_graphs;  // (mode, chunk)

@@ -202,8 +202,9 @@ enum { kWarnVlimit = 0, kWarnForceCap = 1, kWarnConstr = 2, kWarnDxCap = 3, kWar
 // Minimiser (pb2_minimize.cu).  Stage parameters live in device memory
 // (par[kMin*]) so that captured graphs serve every stage.
 enum { kMinK = 0, kMinKind, kMinSdDt, kMinMaxDx, kMinDtStart, kMinDtMax, kMinMaxDisp, kMinForceCap, kMinNPar };
-enum { kMinOpSd = 0, kMinOpRollback, kMinOpFireInit, kMinOpFireBegin, kMinOpFireDrift, kMinOpFireMix,
+enum { kMinOpSd = 0, kMinOpRollback, kMinOpFireInit, kMinOpFireMove, kMinOpFireClose, kMinOpFireEnd,
        kMinOpTakeBest, kMinOpRms };
+constexpr int kMinChunkBlocks = 8;  // 32-atom blocks per chunk: one per warp of a minimiser thread block
 // FIRE constants (Bitzek et al. 2006; jax_md fire_descent defaults)
 constexpr int kFireNmin = 5;
 constexpr double kFireFinc = 1.1, kFireFdec = 0.5, kFireAlphaStart = 0.1, kFireFalpha = 0.99;
@@ -222,6 +223,18 @@ struct MinArgs {
   uint32_t *status;
   const double *par;
   int32_t n_total, n_sys;
+  // thread blocks of the SD and FIRE kernels: (system, its first 32-atom
+  // block) of each chunk, a system's first chunk, and their partial sums
+  const int2 *chunks;
+  const int32_t *chunk0;  // (n_sys + 1)
+  int32_t n_chunks;
+  double *part;           // (n_chunks, 3)
+  int32_t *sys_done;      // chunks arrived; zero between launches
+  double *mix_f, *mix_p;
+  int32_t *sys_flags;
+  float4 *bbox;
+  const float4 *pl_ref;   // as IntArgs
+  int32_t *pl_ctl;
 };
 cudaError_t launch_min(int op, const MinArgs &a, double *out, cudaStream_t st);
 // L-BFGS polish (pb2_minimize.cu)

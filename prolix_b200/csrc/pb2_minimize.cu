@@ -25,8 +25,14 @@
 // uncapped position, and returns the positions of the lowest force RMS seen
 // at the start of an iteration.  The same order is kept here.
 //
-// Per-system sums run in one thread block per system in a fixed order, so
-// the trajectory does not depend on scheduling.
+// An iteration is two launches around the force kernels: min_fire_move (the
+// mixing and cap that close the last iteration, the lowest-RMS snapshot, the
+// half kick and drift) and min_fire_close (the second half kick and the
+// system's sums).  Both run one thread block per 256 atoms; a system's sums
+// are added chunk by chunk in a fixed order by its last block to finish, so
+// the trajectory does not depend on scheduling or on the batch.  (One block
+// per system and four launches took 55 of an iteration's 155 us for 16
+// systems of 150 to 4,000 atoms; these take 9, and an iteration 110.)
 #include "pb2_common.cuh"
 #include "pb2_kernels.cuh"
 
@@ -61,6 +67,19 @@ __device__ __forceinline__ void total_force(const MinArgs &a, int i, double f[3]
     if (!isfinite(f[c])) f[c] = 0.0;
 }
 
+// The float32 copy of atom i's new position (returned for its block's box);
+// raises the pair list's rebuild flag when it is past half the skin.
+__device__ __forceinline__ float4 place_atom(const MinArgs &a, int i, const SysInfo &S, double x, double y, double z) {
+  const float4 q = make_float4((float)(x - S.ox), (float)(y - S.oy), (float)(z - S.oz), (float)a.charge[i]);
+  if (a.pl_ref) {
+    const float4 r = a.pl_ref[i];
+    const float dx = q.x - r.x, dy = q.y - r.y, dz = q.z - r.z;
+    if ((double)fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > S.skin_half2) atomicOr(&a.pl_ctl[PL_DIRTY], 1);
+  }
+  a.posq[i] = q;
+  return q;
+}
+
 __device__ __forceinline__ void put_posq(const MinArgs &a, int i) {
   const SysInfo &S = a.sys[a.atom_sys[i]];
   a.posq[i] = make_float4((float)(a.x[i] - S.ox), (float)(a.y[i] - S.oy), (float)(a.z[i] - S.oz),
@@ -89,24 +108,69 @@ __device__ __forceinline__ void block_sum3(double &v0, double &v1, double &v2) {
   __syncthreads();
 }
 
+// The thread's atom: thread block c is chunk c (system, first 32-atom block
+// of eight), warp w its block w, lane l the block's atom l.
+struct MinAtom {
+  int s, b, i;        // system, batch-wide block, atom
+  bool block, valid;  // the block exists; the atom exists
+};
+__device__ __forceinline__ MinAtom min_atom(const MinArgs &a) {
+  const int2 ch = a.chunks[blockIdx.x];
+  const SysInfo &S = a.sys[ch.x];
+  const int lb = ch.y + (int)(threadIdx.x >> 5);
+  const int l = lb * 32 + (int)(threadIdx.x & 31);
+  return MinAtom{ch.x, S.blk_base + lb, S.off + l, lb < S.nblk, l < S.n};
+}
+
+// Adds the chunk's three sums to its system's; the system's last chunk to
+// arrive gets true in every thread, and the totals, summed in chunk order.
+__device__ __forceinline__ bool sys_sum3(const MinArgs &a, int s, double &v0, double &v1, double &v2) {
+  __shared__ int last;
+  block_sum3(v0, v1, v2);
+  const int c0 = a.chunk0[s], nc = a.chunk0[s + 1] - c0;
+  if (nc == 1) return true;
+  if (threadIdx.x == 0) {
+    double *p = a.part + 3 * (size_t)blockIdx.x;
+    p[0] = v0; p[1] = v1; p[2] = v2;
+    __threadfence();
+    last = atomicAdd(&a.sys_done[s], 1) == nc - 1;
+    if (last) a.sys_done[s] = 0;
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  v0 = v1 = v2 = 0.0;
+  for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+    const double *p = a.part + 3 * (size_t)(c0 + c);
+    v0 += __ldcg(p); v1 += __ldcg(p + 1); v2 += __ldcg(p + 2);
+  }
+  block_sum3(v0, v1, v2);
+  return true;
+}
+
 // ----------------------------------------------------------- steepest descent
 
-__global__ void min_sd_kernel(const MinArgs a) {
+// One warp per 32-atom block, which also writes the block's box.
+__global__ void __launch_bounds__(kMinThreads) min_sd_kernel(const MinArgs a) {
   pdl_wait();
   pdl_trigger();
   const double dt = a.par[kMinSdDt], max_dx = a.par[kMinMaxDx];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
+  const MinAtom m = min_atom(a);
+  if (!m.block) return;
+  float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (m.valid) {
+    const int i = m.i;
     double f[3];
     total_force(a, i, f);
     double d[3] = {f[0] * dt, f[1] * dt, f[2] * dt};
     const double dm = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + 1e-30);
     const double sc = fmin(1.0, max_dx / dm);
-    a.x[i] += d[0] * sc;
-    a.y[i] += d[1] * sc;
-    a.z[i] += d[2] * sc;
+    const double x = a.x[i] + d[0] * sc, y = a.y[i] + d[1] * sc, z = a.z[i] + d[2] * sc;
+    a.x[i] = x; a.y[i] = y; a.z[i] = z;
     a.fx[i] = 0; a.fy[i] = 0; a.fz[i] = 0;
-    put_posq(a, i);
+    q = place_atom(a, i, a.sys[m.s], x, y, z);
   }
+  block_box(a.bbox, m.b, threadIdx.x & 31, m.valid, q);
 }
 
 // A system with any non-finite coordinate goes back to its reference
@@ -134,137 +198,154 @@ __global__ void min_rollback_kernel(const MinArgs a) {
 
 // --------------------------------------------------------------------- FIRE
 
-// p = 0, state force = F + restraint, per-system scalars reset.
-__global__ void min_fire_init_kernel(const MinArgs a) {
+// Scalars that close an iteration, read by the next min_fire_move: p <- p +
+// (mix_f F - mix_p p), or zero; and whether the state force's RMS is the
+// lowest so far.
+enum { kFireZeroP = 1, kFireBetter = 2 };
+
+__device__ __forceinline__ bool rms_is_lowest(const MinArgs &a, int s, double f2) {
+  const double rms = sqrt(f2 / (double)a.sys[s].n);
+  const bool better = rms < a.sys_best[s];
+  if (better) a.sys_best[s] = rms;
+  return better;
+}
+
+// p = 0, state force = F + restraint, per-system scalars reset (a mixing that
+// changes nothing pending).
+__global__ void __launch_bounds__(kMinThreads) min_fire_init_kernel(const MinArgs a) {
   const size_t N = a.n_total;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
+  const MinAtom m = min_atom(a);
+  double f2 = 0.0, z0 = 0.0, z1 = 0.0;
+  if (m.valid) {
+    const int i = m.i;
     double f[3];
     total_force(a, i, f);
     a.ft[i] = f[0]; a.ft[N + i] = f[1]; a.ft[2 * N + i] = f[2];
     a.px[i] = 0.0; a.py[i] = 0.0; a.pz[i] = 0.0;
-    a.best[i] = a.x[i]; a.best[N + i] = a.y[i]; a.best[2 * N + i] = a.z[i];
+    const double x = a.x[i], y = a.y[i], z = a.z[i];
+    a.best[i] = x; a.best[N + i] = y; a.best[2 * N + i] = z;
+    a.xb[i] = x; a.xb[N + i] = y; a.xb[2 * N + i] = z;
+    f2 = f[0] * f[0] + f[1] * f[1] + f[2] * f[2];
   }
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < a.n_sys; s += gridDim.x * blockDim.x) {
-    a.sys_dt[s] = a.par[kMinDtStart];
-    a.sys_alpha[s] = kFireAlphaStart;
-    a.sys_npos[s] = 0;
-    a.sys_best[s] = 1e10;
-  }
-}
-
-// Start of an iteration: RMS of the state force; keep the positions if it is
-// the lowest so far.
-__global__ void min_fire_begin_kernel(const MinArgs a) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ int better;
-  const size_t N = a.n_total;
-  for (int s = blockIdx.x; s < a.n_sys; s += gridDim.x) {
-    const SysInfo &S = a.sys[s];
-    double f2 = 0.0, z0 = 0.0, z1 = 0.0;
-    for (int i = S.off + threadIdx.x; i < S.off + S.n; i += blockDim.x)
-      f2 += a.ft[i] * a.ft[i] + a.ft[N + i] * a.ft[N + i] + a.ft[2 * N + i] * a.ft[2 * N + i];
-    block_sum3(f2, z0, z1);
-    if (threadIdx.x == 0) {
-      const double rms = sqrt(f2 / (double)S.n);
-      better = rms < a.sys_best[s];
-      if (better) a.sys_best[s] = rms;
-    }
-    __syncthreads();
-    if (better)
-      for (int i = S.off + threadIdx.x; i < S.off + S.n; i += blockDim.x) {
-        a.best[i] = a.x[i]; a.best[N + i] = a.y[i]; a.best[2 * N + i] = a.z[i];
-      }
-    __syncthreads();
+  if (sys_sum3(a, m.s, f2, z0, z1) && threadIdx.x == 0) {
+    a.sys_dt[m.s] = a.par[kMinDtStart];
+    a.sys_alpha[m.s] = kFireAlphaStart;
+    a.sys_npos[m.s] = 0;
+    a.sys_best[m.s] = 1e10;
+    a.mix_f[m.s] = 0.0;
+    a.mix_p[m.s] = 0.0;
+    a.sys_flags[m.s] = rms_is_lowest(a, m.s, f2) ? kFireBetter : 0;
   }
 }
 
-// First half kick and drift; remembers the positions for the displacement
-// cap.  With a force cap (prolix simulate.py:613-621) the state force of
-// each atom is scaled to at most that norm for this kick.
-__global__ void min_fire_drift_kernel(const MinArgs a) {
+// The mixing and the displacement cap that close the last iteration.
+__device__ __forceinline__ void close_iteration(const MinArgs &a, int i, int s, int flags, double x[3], double p[3],
+                                                const double f[3]) {
+  const size_t N = a.n_total;
+  const double max_disp = a.par[kMinMaxDisp], mf = a.mix_f[s], mp = a.mix_p[s];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) p[c] = (flags & kFireZeroP) ? 0.0 : p[c] + (mf * f[c] - mp * p[c]);
+  const double xb[3] = {a.xb[i], a.xb[N + i], a.xb[2 * N + i]};
+  const double dx = x[0] - xb[0], dy = x[1] - xb[1], dz = x[2] - xb[2];
+  const double dm = sqrt(dx * dx + dy * dy + dz * dz + 1e-30);
+  const double sc = max_disp > 0.0 ? fmin(1.0, max_disp / dm) : 1.0;  // 0: no cap
+  x[0] = xb[0] + dx * sc; x[1] = xb[1] + dy * sc; x[2] = xb[2] + dz * sc;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) p[c] *= sc;
+}
+
+// Start of an iteration: closes the last one, keeps the positions if their
+// force RMS is the lowest so far, then the first half kick and drift; the
+// positions before are remembered for the displacement cap.  With a force cap
+// (prolix simulate.py:613-621) the state force of each atom is scaled to at
+// most that norm for this kick.  Also writes the blocks' boxes.
+__global__ void __launch_bounds__(kMinThreads) min_fire_move_kernel(const MinArgs a) {
   pdl_wait();
   pdl_trigger();
   const size_t N = a.n_total;
-  const double cap = a.par[kMinForceCap];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total; i += gridDim.x * blockDim.x) {
-    const double dt = a.sys_dt[a.atom_sys[i]], h = 0.5 * dt, m = a.mass[i];
+  const MinAtom m = min_atom(a);
+  if (!m.block) return;
+  float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (m.valid) {
+    const int i = m.i;
+    const int flags = a.sys_flags[m.s];
+    const double cap = a.par[kMinForceCap], dt = a.sys_dt[m.s], h = 0.5 * dt, ms = a.mass[i];
     double f[3] = {a.ft[i], a.ft[N + i], a.ft[2 * N + i]};
+    double x[3] = {a.x[i], a.y[i], a.z[i]}, p[3] = {a.px[i], a.py[i], a.pz[i]};
+    close_iteration(a, i, m.s, flags, x, p, f);
+    if (flags & kFireBetter) {
+      a.best[i] = x[0]; a.best[N + i] = x[1]; a.best[2 * N + i] = x[2];
+    }
     if (cap > 0.0) {
       const double sc = fmin(1.0, cap / (sqrt(f[0] * f[0] + f[1] * f[1] + f[2] * f[2]) + 1e-8));
       f[0] *= sc; f[1] *= sc; f[2] *= sc;
     }
-    const double px = a.px[i] + h * f[0], py = a.py[i] + h * f[1], pz = a.pz[i] + h * f[2];
+    const double px = p[0] + h * f[0], py = p[1] + h * f[1], pz = p[2] + h * f[2];
     a.px[i] = px; a.py[i] = py; a.pz[i] = pz;
-    a.xb[i] = a.x[i]; a.xb[N + i] = a.y[i]; a.xb[2 * N + i] = a.z[i];
-    a.x[i] += dt * px / m;
-    a.y[i] += dt * py / m;
-    a.z[i] += dt * pz / m;
+    a.xb[i] = x[0]; a.xb[N + i] = x[1]; a.xb[2 * N + i] = x[2];
+    x[0] += dt * px / ms;
+    x[1] += dt * py / ms;
+    x[2] += dt * pz / ms;
+    a.x[i] = x[0]; a.y[i] = x[1]; a.z[i] = x[2];
     a.fx[i] = 0; a.fy[i] = 0; a.fz[i] = 0;
-    put_posq(a, i);
+    q = place_atom(a, i, a.sys[m.s], x[0], x[1], x[2]);
   }
+  block_box(a.bbox, m.b, threadIdx.x & 31, m.valid, q);
 }
 
-// Second half kick with the new force, FIRE mixing and time-step control,
-// then the displacement cap.
-__global__ void min_fire_mix_kernel(const MinArgs a) {
+// Second half kick with the new force, and the system's sums: the FIRE mixing
+// factors and time-step control, and the RMS of the new state force.
+__global__ void __launch_bounds__(kMinThreads) min_fire_close_kernel(const MinArgs a) {
   pdl_wait();
   pdl_trigger();
-  __shared__ double mix_f, mix_p;
-  __shared__ int zero_p;
   const size_t N = a.n_total;
-  const double max_disp = a.par[kMinMaxDisp], dt_max = a.par[kMinDtMax];
-  for (int s = blockIdx.x; s < a.n_sys; s += gridDim.x) {
-    const SysInfo &S = a.sys[s];
+  const MinAtom m = min_atom(a);
+  const int s = m.s;
+  const double dt_max = a.par[kMinDtMax];
+  double fp = 0.0, f2 = 0.0, p2 = 0.0;
+  if (m.valid) {
+    const int i = m.i;
     const double h = 0.5 * a.sys_dt[s];
-    double fp = 0.0, f2 = 0.0, p2 = 0.0;
-    for (int i = S.off + threadIdx.x; i < S.off + S.n; i += blockDim.x) {
-      double f[3];
-      total_force(a, i, f);
-      a.ft[i] = f[0]; a.ft[N + i] = f[1]; a.ft[2 * N + i] = f[2];
-      const double px = a.px[i] + h * f[0], py = a.py[i] + h * f[1], pz = a.pz[i] + h * f[2];
-      a.px[i] = px; a.py[i] = py; a.pz[i] = pz;
-      fp += f[0] * px + f[1] * py + f[2] * pz;
-      f2 += f[0] * f[0] + f[1] * f[1] + f[2] * f[2];
-      p2 += px * px + py * py + pz * pz;
-    }
-    block_sum3(fp, f2, p2);
-    if (threadIdx.x == 0) {
-      const double alpha = a.sys_alpha[s];
-      const double fn = sqrt(f2 + 1e-6), pn = sqrt(p2);
-      mix_f = alpha * pn / fn;
-      mix_p = alpha;
-      int npos = fp >= 0.0 ? a.sys_npos[s] + 1 : 0;
-      double dt = a.sys_dt[s], al = alpha;
-      if (fp > 0.0 && npos > kFireNmin) {
-        dt = fmin(dt * kFireFinc, dt_max);
-        al = al * kFireFalpha;
-      }
-      if (fp < 0.0) {
-        dt = dt * kFireFdec;
-        al = kFireAlphaStart;
-      }
-      zero_p = fp < 0.0;
-      a.sys_npos[s] = npos;
-      a.sys_dt[s] = dt;
-      a.sys_alpha[s] = al;
-    }
-    __syncthreads();
-    for (int i = S.off + threadIdx.x; i < S.off + S.n; i += blockDim.x) {
-      double p[3] = {a.px[i], a.py[i], a.pz[i]};
-      const double f[3] = {a.ft[i], a.ft[N + i], a.ft[2 * N + i]};
-#pragma unroll
-      for (int c = 0; c < 3; ++c) p[c] = zero_p ? 0.0 : p[c] + (mix_f * f[c] - mix_p * p[c]);
-      const double dx = a.x[i] - a.xb[i], dy = a.y[i] - a.xb[N + i], dz = a.z[i] - a.xb[2 * N + i];
-      const double dm = sqrt(dx * dx + dy * dy + dz * dz + 1e-30);
-      const double sc = max_disp > 0.0 ? fmin(1.0, max_disp / dm) : 1.0;  // 0: no cap
-      a.x[i] = a.xb[i] + dx * sc;
-      a.y[i] = a.xb[N + i] + dy * sc;
-      a.z[i] = a.xb[2 * N + i] + dz * sc;
-      a.px[i] = p[0] * sc; a.py[i] = p[1] * sc; a.pz[i] = p[2] * sc;
-    }
-    __syncthreads();
+    double f[3];
+    total_force(a, i, f);
+    a.ft[i] = f[0]; a.ft[N + i] = f[1]; a.ft[2 * N + i] = f[2];
+    const double px = a.px[i] + h * f[0], py = a.py[i] + h * f[1], pz = a.pz[i] + h * f[2];
+    a.px[i] = px; a.py[i] = py; a.pz[i] = pz;
+    fp = f[0] * px + f[1] * py + f[2] * pz;
+    f2 = f[0] * f[0] + f[1] * f[1] + f[2] * f[2];
+    p2 = px * px + py * py + pz * pz;
   }
+  if (!sys_sum3(a, s, fp, f2, p2) || threadIdx.x != 0) return;
+  const double alpha = a.sys_alpha[s];
+  a.mix_f[s] = alpha * sqrt(p2) / sqrt(f2 + 1e-6);
+  a.mix_p[s] = alpha;
+  const int npos = fp >= 0.0 ? a.sys_npos[s] + 1 : 0;
+  double dt = a.sys_dt[s], al = alpha;
+  if (fp > 0.0 && npos > kFireNmin) {
+    dt = fmin(dt * kFireFinc, dt_max);
+    al = al * kFireFalpha;
+  }
+  if (fp < 0.0) {
+    dt = dt * kFireFdec;
+    al = kFireAlphaStart;
+  }
+  a.sys_npos[s] = npos;
+  a.sys_dt[s] = dt;
+  a.sys_alpha[s] = al;
+  a.sys_flags[s] = (fp < 0.0 ? kFireZeroP : 0) | (rms_is_lowest(a, s, f2) ? kFireBetter : 0);
+}
+
+// End of a FIRE stage: closes its last iteration.
+__global__ void __launch_bounds__(kMinThreads) min_fire_end_kernel(const MinArgs a) {
+  const size_t N = a.n_total;
+  const MinAtom m = min_atom(a);
+  if (!m.valid) return;
+  const int i = m.i;
+  const double f[3] = {a.ft[i], a.ft[N + i], a.ft[2 * N + i]};
+  double x[3] = {a.x[i], a.y[i], a.z[i]}, p[3] = {a.px[i], a.py[i], a.pz[i]};
+  close_iteration(a, i, m.s, a.sys_flags[m.s], x, p, f);
+  a.x[i] = x[0]; a.y[i] = x[1]; a.z[i] = x[2];
+  a.px[i] = p[0]; a.py[i] = p[1]; a.pz[i] = p[2];
 }
 
 // End of a FIRE stage: the best positions become the state.
@@ -481,12 +562,12 @@ cudaError_t launch_min(int op, const MinArgs &a, double *out, cudaStream_t st) {
   if (a.n_total <= 0) return cudaSuccess;
   const int ga = atom_grid(a.n_total), gs = a.n_sys;
   switch (op) {
-    case kMinOpSd: return launch_after(min_sd_kernel, ga, kMinThreads, st, a);
+    case kMinOpSd: return launch_after(min_sd_kernel, a.n_chunks, kMinThreads, st, a);
     case kMinOpRollback: min_rollback_kernel<<<gs, kMinThreads, 0, st>>>(a); break;
-    case kMinOpFireInit: min_fire_init_kernel<<<ga, kMinThreads, 0, st>>>(a); break;
-    case kMinOpFireBegin: return launch_after(min_fire_begin_kernel, gs, kMinThreads, st, a);
-    case kMinOpFireDrift: return launch_after(min_fire_drift_kernel, ga, kMinThreads, st, a);
-    case kMinOpFireMix: return launch_after(min_fire_mix_kernel, gs, kMinThreads, st, a);
+    case kMinOpFireInit: min_fire_init_kernel<<<a.n_chunks, kMinThreads, 0, st>>>(a); break;
+    case kMinOpFireMove: return launch_after(min_fire_move_kernel, a.n_chunks, kMinThreads, st, a);
+    case kMinOpFireClose: return launch_after(min_fire_close_kernel, a.n_chunks, kMinThreads, st, a);
+    case kMinOpFireEnd: min_fire_end_kernel<<<a.n_chunks, kMinThreads, 0, st>>>(a); break;
     case kMinOpTakeBest: min_take_best_kernel<<<ga, kMinThreads, 0, st>>>(a); break;
     case kMinOpRms: min_rms_kernel<<<gs, kMinThreads, 0, st>>>(a, out); break;
     default: return cudaErrorInvalidValue;
