@@ -980,6 +980,19 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   if (!(params->terms & (PB2_USE_LJ | PB2_USE_COULOMB))) B.n_exc = 0;
 
   b->grid_bonded = 8 * ctx->sm_count;
+  {
+    // A batch of at most two waves of single tiles: thread blocks of four
+    // warps spread them more evenly over the SMs than eight, and the
+    // descreening pass runs faster with the registers of two resident blocks
+    // than with a third (us per step with the larger batches' shapes and
+    // these: 1,800 atoms 40.1, 36.1; 2,500 at 20 A 52.5, 47.4; 4,000 71.2,
+    // 66.9; 6,000, 8,930 tiles 114.0, 113.7; 256 ragged systems 1313, 1341).
+    long long tiles = 0;
+    for (const SysInfo &S : sinfo)
+      for (int ib = 0; ib < S.nblk; ib += 2) tiles += S.nblk - ib;
+    if (tiles <= 2LL * 16 * ctx->sm_count)
+      for (int &sh : b->shape) sh = 1;
+  }
   if ((rc = setup_items2(b.get(), b->params.tile_segment))) return rc;
   if ((rc = setup_pair_list(b.get(), b->params.tile_segment))) return rc;
   {

@@ -1457,7 +1457,7 @@ __global__ void bbox_kernel(const SysInfo *sys, const int32_t *blk_sys, const fl
 // --------------------------------------------------------------- launchers
 
 // Block shapes compiled for each pass (threads, min blocks per SM); entry 0
-// is the default.  The descreening pass holds fewer registers, so its
+// is the default of batches of many tiles, entry 1 of batches of few.  The descreening pass holds fewer registers, so its
 // shapes allow more resident blocks.
 struct Shape {
   int threads, minb;
