@@ -222,7 +222,10 @@ int pb2_born_radii(pb2_batch *batch, double *born, void *stream);
  * (n_atoms_total, 3), row-major FP64, either may be NULL.  Asynchronous on
  * `stream`; allocates and synchronises nothing, so an XLA FFI handler (the
  * binding a prolix maintainer adds for make_energy_fn, system.py:29-271)
- * or a captured CUDA graph can call it. */
+ * or a captured CUDA graph can call it.  The energies run on a stream of the
+ * batch forked from `stream` and joined to it; from the third call on (outside
+ * a capture) a small batch's launches are replayed as a CUDA graph,
+ * instantiated then. */
 int pb2_energy_forces_device(pb2_batch *batch, const double *positions, double *energies,
                              double *forces, void *stream);
 

@@ -134,6 +134,11 @@ struct pb2_batch {
   int grid_team[3] = {1, 1, 1};
   cudaStream_t cap_stream = nullptr;
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
+  // evaluations without and with energies: graph, and calls before it
+  cudaGraphExec_t eval_graphs[2] = {nullptr, nullptr};
+  int evals[2] = {0, 0};
+  cudaStream_t side = nullptr;  // the FP64 energies of an evaluation, beside its forces
+  cudaEvent_t ev_side[2] = {nullptr, nullptr};
   bool profiling = false;
   double timings[kTimSlots] = {0, 0, 0, 0, 0, 0, 0, 0};
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -182,10 +187,24 @@ struct pb2_batch {
   cudaEvent_t nl_ev[2] = {nullptr, nullptr};  // around the last build's launches
   bool nl_timed = false;
 
-  ~pb2_batch() {
+  // Every captured graph (their kernels, shapes and work lists are fixed).
+  void drop_graphs() {
     for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
+    graphs.clear();
     for (auto &kv : min_graphs) cudaGraphExecDestroy(kv.second);
+    min_graphs.clear();
+    for (auto &g : eval_graphs) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
+  }
+
+  ~pb2_batch() {
+    drop_graphs();
     if (cap_stream) cudaStreamDestroy(cap_stream);
+    if (side) cudaStreamDestroy(side);
+    for (auto &e : ev_side)
+      if (e) cudaEventDestroy(e);
     for (auto &e : ev)
       if (e) cudaEventDestroy(e);
     for (auto &e : ev_io)
