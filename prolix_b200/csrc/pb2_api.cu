@@ -83,6 +83,7 @@ static PairArgs pair_args(pb2_batch *b) {
   a.cut = b->cut ? 1 : 0;
   a.sched = b->sched;
   a.early = 0;
+  a.heads = 0;
   a.born_acc = b->born_acc;
   a.dedb_acc = b->dedb_acc;
   a.fx = b->fx;
@@ -1087,6 +1088,11 @@ static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_ene
     // the descreening pass finalizes each block once its system's items are
     // summed (profiling keeps the separate launch, to time it)
     const bool fuse_finalize = !b->profiling && (b->fuse & PB2_FUSE_FINALIZE);
+    // teams for all three passes: no finalize launch (profiling keeps it)
+    if (b->team && !fuse_finalize && !b->profiling && (b->force_blocks == 2 || b->pl_on)) {
+      pa.heads = 1;
+      pa.fin = fa;
+    }
     PairArgs pb = pa;
     pb.sched = b->sched + 2 * PASS_BORN;
     if (fuse_finalize) {
@@ -1094,7 +1100,7 @@ static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_ene
       pb.fin = fa;
     }
     if ((e = tm(kTimBorn, [&] { return enqueue_pass(b, PASS_BORN, pb, st); })) != cudaSuccess) return e;
-    if (!fuse_finalize &&
+    if (!fuse_finalize && !pa.heads &&
         (e = tm(kTimFinalize, [&] { return launch_born_finalize(fa, st); })) != cudaSuccess)
       return e;
   }

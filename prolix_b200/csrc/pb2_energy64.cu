@@ -290,6 +290,7 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
   M.use_coul = (a.terms & PB2_USE_COULOMB) != 0;
   const bool all_terms = M.use_gb && M.use_lj && M.use_coul;
   const uint32_t diag_mask = lane == 31 ? 0u : (0xffffffffu << (lane + 1));
+  const bool one_wave = a.n_items <= nwarps;  // no warp asks the counter for another item
   pdl_wait();
   pdl_trigger();
   for (int it = wl * (int)gridDim.x + (int)blockIdx.x; it < a.n_items;) {
@@ -420,12 +421,13 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
     } else {
       flush_energy64(a, item.sys, e_gb, e_coul, e_lj, lane);
     }
+    if (one_wave) break;
     int next = 0;
     if (lane == 0) next = nwarps + atomicAdd(&a.sched[0], 1);
     it = __shfl_sync(kFull, next, 0);
   }
   if (PASS == 0 && Q.n > 0) e64_drain(a, Q, lane);
-  if (lane == 0 && atomicAdd(&a.sched[1], 1) == nwarps - 1) {
+  if (!one_wave && lane == 0 && atomicAdd(&a.sched[1], 1) == nwarps - 1) {
     // every warp has stopped taking items: reset for the next launch
     a.sched[0] = 0;
     a.sched[1] = 0;

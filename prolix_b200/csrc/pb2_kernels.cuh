@@ -75,6 +75,7 @@ struct PairArgs {
   long long *energy;
   int32_t cut;              // any cutoff active
   int32_t *sched;           // (next item, finished warps) of this pass; zero between launches
+  int32_t heads;            // team kernels: the force pass makes the Born radii (no finalize launch); fin is set
   int32_t early;            // 1: the positions and boxes are older than the launch before this one
   // pair list (cutoff runs; NULL otherwise): items come from pl_items[pl_ctl[1]],
   // pl_ctl[2 + pl_ctl[1]] of them, and an item's tiles t in [jb0, jb1) are

@@ -184,11 +184,12 @@ __device__ __forceinline__ void load_pos(const PairArgs &a, int g, PData &P) {
   const float4 p = a.posq[g];
   P.x = p.x; P.y = p.y; P.z = p.z; P.q = p.w;
 }
-// The Born data (after load_par).
-__device__ __forceinline__ void load_born(const PairArgs &a, int g, int pass, bool use_gb, PData &P) {
+// The Born data (after load_par); own: from there, not from a.born.
+__device__ __forceinline__ void load_born(const PairArgs &a, int g, int pass, bool use_gb, PData &P,
+                                          const float4 *own = nullptr) {
   P.B = P.iB = P.dedi = P.rB = 0.f;
   if ((pass == PASS_FORCE && use_gb) || pass == PASS_CHAIN) {
-    const float4 b = a.born[g];
+    const float4 b = own ? *own : a.born[g];
     P.B = b.x; P.iB = b.y * kSqrtQuarterLog2e; P.rB = b.y;
     if (pass == PASS_CHAIN) P.dedi = (float)((double)a.dedb_acc[g] * kForceInv) * b.z;
   }
@@ -603,16 +604,19 @@ __device__ __forceinline__ void run_bc_tile2(const PData2 &I, const JTile &jt, A
 
 // One atom's Born radius from its descreening sum, and the per-atom GB
 // self term and ACE as the initial dE/dB; clears the sum.
+__device__ __forceinline__ long long self_dedb(const FinalizeArgs &a, int i, const SysInfo &S, double r_in,
+                                               const BornRadius &R) {
+  const double q = a.charge[i];
+  const double ace = ace_energy(r_in, R.B);
+  return to_fix(-S.pref_d * q * q * R.inv_b * R.inv_b - 6.0 * ace * R.inv_b, kForceScale);
+}
 __device__ __forceinline__ void finalize_atom(const FinalizeArgs &a, int i, const SysInfo &S) {
   const double isum = (double)__ldcg(&a.born_acc[i]) * kBornInv;
   a.born_acc[i] = 0;
   const double r_in = a.radius[i];
   const BornRadius R = born_radius(isum, r_in, S.clamp != 0);
   a.born[i] = make_float4((float)R.B, (float)R.inv_b, (float)R.dbdi, 0.f);
-  const double q = a.charge[i];
-  const double ace = ace_energy(r_in, R.B);
-  const double dedb = -S.pref_d * q * q * R.inv_b * R.inv_b - 6.0 * ace * R.inv_b;
-  a.dedb_acc[i] = to_fix(dedb, kForceScale);
+  a.dedb_acc[i] = self_dedb(a, i, S, r_in, R);
 }
 
 // Spins of the bounded waits (each a 128 ns sleep and an L2 read): about a
@@ -729,10 +733,13 @@ __global__ void __launch_bounds__(THREADS, MINB)
   // finalize waits for items: there every item comes from the counter, so
   // that each one waited for was taken by a running warp.
   const bool counted = PASS == PASS_BORN && sys_items;
+  // an item for every warp: none asks the counter for another
+  const bool one_wave = !counted && n_items + (PASS == PASS_CHAIN ? a.n_bonded_chunks : 0) <= nwarps;
   const int base = counted ? 0 : nwarps;
   int it = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
   for (bool own = !counted;; own = false) {
     if (!own) {
+      if (one_wave) break;
       if (lane == 0) it = base + atomicAdd(&a.sched[0], 1);
       it = __shfl_sync(kFull, it, 0);
     }
@@ -922,7 +929,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
   if constexpr (PASS != PASS_FORCE) {
     if (Q.n > 0) cf_drain<PASS>(Q, lane);
   }
-  if (lane == 0 && atomicAdd(&a.sched[1], 1) == nwarps - 1) {
+  if (!one_wave && lane == 0 && atomicAdd(&a.sched[1], 1) == nwarps - 1) {
     // every warp has stopped taking items: reset for the next launch
     a.sched[0] = 0;
     a.sched[1] = 0;
@@ -943,6 +950,9 @@ __global__ void __launch_bounds__(THREADS, MINB)
 // differently, and kept so in large batches they cost those 5 to 10 %.)
 // us per step with one warp per tile and with teams: 166 atoms 34.2, 20.9;
 // 896 atoms 36.9, 22.5.
+// With a.heads there is no finalize launch between the descreening and force
+// passes: each force tile turns its three blocks' sums into Born radii, three
+// warps side by side (166 atoms 20.8 -> 18.8, 1,500 30.2 -> 29.5).
 
 // A tile in shared memory.  Entry k * 32 + l of the factors is lane l's at
 // step k: (g, h) of the force pass in g4; (vij, vji) of the descreening pass
@@ -953,6 +963,7 @@ struct TeamShared {
   float2 ix[3][32];                            // the i atoms' packed positions
   float2 rb[32];                               // their 1 / B
   float jrb[32];
+  float4 born[PASS == PASS_FORCE ? 3 : 1][32];  // a.heads: the j and both i blocks' Born data
   float4 g4[PASS == PASS_CHAIN ? 1 : 1024];
   float2 g2[PASS == PASS_FORCE ? 1 : 1024];
   int next;
@@ -1067,6 +1078,9 @@ __global__ void __launch_bounds__(32 * W) team_kernel(const __grid_constant__ Pa
   }
   // units: W bonded chunks each (the longest), then the items
   const int n_bonded = PASS == PASS_CHAIN ? (a.n_bonded_chunks + W - 1) / W : 0;
+  // a unit for every block: none asks the counter for another (a round trip
+  // to L2 at the end of the kernel)
+  const bool one_wave = n_bonded + n_items <= (int)gridDim.x;
   for (int u = (int)blockIdx.x; u < n_bonded + n_items;) {
     if (u < n_bonded) {
       const int t = (u * W + w) * kBondedChunk + lane;
@@ -1126,9 +1140,37 @@ __global__ void __launch_bounds__(32 * W) team_kernel(const __grid_constant__ Pa
           if (PASS == PASS_FORCE) reach2 = (K.gcut2 == 0.f || K.cut2 == 0.f) ? 0.f : fmaxf(K.gcut2, K.cut2);
           if (reach2 > 0.f && d2 >= reach2) continue;  // no pair within reach (block-uniform)
         }
-        load_born(a, ig0, PASS, K.use_gb, I0);
-        load_born(a, ig1, PASS, K.use_gb, I1);
-        load_born(a, jg, PASS, K.use_gb, J);
+        if (PASS == PASS_FORCE && a.heads) {
+          // Born radii from the descreening sums, a warp per block of the
+          // tile; a block's diagonal tile also writes them out and adds its
+          // atoms' self terms
+          if constexpr (PASS == PASS_FORCE) {
+            if (w < 3) {
+              const int g = w == 0 ? jg : w == 1 ? ig0 : ig1;
+              const double r_in = a.fin.radius[g];
+              const BornRadius B = born_radius((double)__ldcg(&a.born_acc[g]) * kBornInv, r_in, S.clamp != 0);
+              const float4 b = make_float4((float)B.B, (float)B.inv_b, (float)B.dbdi, 0.f);
+              T.born[w][lane] = b;
+              if (w == 0 && jvalid && (jb == ib0 || jb == ib1)) {
+                a.fin.born[g] = b;
+                atomic_add_fix(&a.dedb_acc[g], self_dedb(a.fin, g, S, r_in, B));
+              }
+            }
+            __syncthreads();
+            load_born(a, ig0, PASS, true, I0, &T.born[1][lane]);
+            load_born(a, ig1, PASS, true, I1, &T.born[2][lane]);
+            load_born(a, jg, PASS, true, J, &T.born[0][lane]);
+          }
+        } else {
+          load_born(a, ig0, PASS, K.use_gb, I0);
+          load_born(a, ig1, PASS, K.use_gb, I1);
+          load_born(a, jg, PASS, K.use_gb, J);
+          // without a finalize launch: the descreening pass clears dE/dB for
+          // the force pass, the chain pass the descreening sums for the next
+          // evaluation, each at its blocks' diagonal tiles
+          if (PASS != PASS_FORCE && a.heads && w == 0 && jvalid && (jb == ib0 || jb == ib1))
+            (PASS == PASS_BORN ? a.dedb_acc : a.born_acc)[jg] = 0;
+        }
         if (w == 0) {
           store_j<PASS>(T.jt, lane, J);
           T.jrb[lane] = J.rB;
@@ -1224,13 +1266,14 @@ __global__ void __launch_bounds__(32 * W) team_kernel(const __grid_constant__ Pa
         __syncthreads();  // the tile's shared data are read before the next tile's are written
       }
     }
+    if (one_wave) break;
     if (threadIdx.x == 0) T.next = (int)gridDim.x + atomicAdd(&a.sched[0], 1);
     __syncthreads();
     u = T.next;
     __syncthreads();
   }
   if (!waited) pdl_wait();
-  if (threadIdx.x == 0 && atomicAdd(&a.sched[1], 1) == (int)gridDim.x - 1) {
+  if (!one_wave && threadIdx.x == 0 && atomicAdd(&a.sched[1], 1) == (int)gridDim.x - 1) {
     a.sched[0] = 0;
     a.sched[1] = 0;
   }
