@@ -260,28 +260,37 @@ static std::vector<TileItem> build_items2(const std::vector<SysInfo> &sinfo, int
 
 // Items of the FP64 energy kernels: pairs of i-blocks.  Each item's sums are
 // rounded to fixed point once, so how a system is cut depends on its own size
-// alone and its energies are the same in every batch.  A small system has
-// its tiles' 32 steps shared by 8, 4 or 2 items (as many as one resident
-// wave of 1,776 warps holds): what it waits for is its longest item.  A large
-// one takes several tiles per item, which load their i atoms once.
-static std::vector<TileItem> build_items_e64(const std::vector<SysInfo> &sinfo) {
-  std::vector<TileItem> items;
+// alone and its energies are the same in every batch.  A small system (up to
+// 57 blocks, 870 tiles) waits for its longest item: its tiles' 32 steps are
+// shared by 8, 4 or 2 items in the descreening pass (as many as one resident
+// wave of 1,776 warps holds), and by a thread block's warps in the energy
+// pass (tiles).  A large one takes several tiles per item, which load their i
+// atoms once.
+struct E64Items {
+  std::vector<TileItem> born, pair, tiles;
+};
+static E64Items build_items_e64(const std::vector<SysInfo> &sinfo) {
+  E64Items out;
   for (int s = 0; s < (int)sinfo.size(); ++s) {
     const int nblk = sinfo[s].nblk;
     const int parts = nblk <= 28 ? 8 : nblk <= 40 ? 4 : nblk <= 57 ? 2 : 1;  // 224, 440, 870 tiles
     const int seg = nblk < 160 ? 1 : nblk < 256 ? 2 : nblk < 400 ? 4 : 8;
     const int kn = 32 / parts;
     for (int ib = 0; ib < nblk; ib += 2)
-      for (int j0 = ib; j0 < nblk; j0 += seg)
+      for (int j0 = ib; j0 < nblk; j0 += seg) {
+        const TileItem whole{s, ib, j0, std::min(j0 + seg, nblk)};
         for (int p = 0; p < parts; ++p)
-          items.push_back(TileItem{s, ib, j0, parts > 1 ? part_code(p * kn, kn) : std::min(j0 + seg, nblk)});
+          out.born.push_back(parts > 1 ? TileItem{s, ib, j0, part_code(p * kn, kn)} : whole);
+        (parts > 1 ? out.tiles : out.pair).push_back(whole);
+      }
   }
   auto cost = [](const TileItem &t) {
     const ItemRange r = item_range(t);
     return (r.jb1 - r.jb0) * r.kn;
   };
-  std::stable_sort(items.begin(), items.end(), [&](const TileItem &p, const TileItem &q) { return cost(p) > cost(q); });
-  return items;
+  for (auto *v : {&out.born, &out.pair})
+    std::stable_sort(v->begin(), v->end(), [&](const TileItem &p, const TileItem &q) { return cost(p) > cost(q); });
+  return out;
 }
 
 // Work items of the four-block force kernel: i-blocks ib, ib % 4 == 0 (with
@@ -601,7 +610,7 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   std::vector<int32_t> hblk_sys(blocks_total);
   std::vector<int4> hblk_info(blocks_total);
   std::vector<ExclRow> hrows;
-  std::vector<TileItem> hitems;
+  E64Items he64;
   int blk_base = 0;
   for (int s = 0; s < n_systems; ++s) {
     const pb2_system_desc &d = systems[s];
@@ -741,10 +750,14 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
     blk_base += S.nblk;
   }
   {
-    hitems = build_items_e64(sinfo);
-    b->n_items = (int)hitems.size();
+    he64 = build_items_e64(sinfo);
+    b->n_items = (int)he64.born.size();
+    b->n_items_e = (int)he64.pair.size();
+    b->n_tiles_e = (int)he64.tiles.size();
+    const int n[2] = {b->n_items, b->n_items_e};
     for (int p = 0; p < 2; ++p)
-      b->grid_e64[p] = std::max(1, std::min(energy64_occupancy(p) * ctx->sm_count, b->n_items));
+      b->grid_e64[p] = std::max(1, std::min(energy64_occupancy(p) * ctx->sm_count, n[p]));
+    b->grid_tiles_e = std::max(1, std::min(energy64_tile_occupancy() * ctx->sm_count, b->n_tiles_e));
   }
   b->sys_host = sinfo;
 
@@ -881,12 +894,12 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
     b->pl_on = finite && (direct || gbt) && many;
     b->pl_reach2 = (float)((reach + params->skin) * (reach + params->skin));
   }
-  b->q64 = D.alloc<double>(N);
   b->hs64 = D.alloc<double>(N);
   b->se64 = D.alloc<double>(N);
   b->ro64 = D.alloc<double>(N);
   b->sr64 = D.alloc<double>(N);
   b->born64 = D.alloc<double>(N);
+  b->iborn64 = D.alloc<double>(N);
   b->stage = D.alloc<double>(9 * (size_t)N);  // x, p, F rows of a host round trip
   b->user = D.alloc<int32_t>(N);
   b->devidx = D.alloc<int32_t>(N);
@@ -901,7 +914,9 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   b->guard_end = D.alloc<int32_t>(1);
   b->warn_flags = D.alloc<uint32_t>(2 * (size_t)n_systems);
   b->warn_counts = D.alloc<int32_t>((size_t)n_systems * kWarnTypes);
-  b->items = D.alloc<TileItem>(hitems.size());
+  b->items = D.alloc<TileItem>(he64.born.size());
+  b->items_e = D.alloc<TileItem>(he64.pair.size());
+  b->tiles_e = D.alloc<TileItem>(he64.tiles.size());
   b->excl_ent = D.alloc<int2>(hent.size());
   b->excl_rows = D.alloc<ExclRow>(hrows.size());
   BondedArgs &B = b->bonded;
@@ -934,12 +949,13 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
       (rc = upload(ctx, b->mass, hm)) || (rc = upload(ctx, b->sigma, hsig)) ||
       (rc = upload(ctx, b->charge, hq)) || (rc = upload(ctx, b->radius, hrad)) ||
       (rc = upload(ctx, b->posq, hposq)) || (rc = upload(ctx, b->par, hpar)) ||
-      (rc = upload(ctx, b->q64, hq)) || (rc = upload(ctx, b->hs64, hhs)) ||
+      (rc = upload(ctx, b->hs64, hhs)) ||
       (rc = upload(ctx, b->se64, hse)) || (rc = upload(ctx, b->ro64, hro)) ||
       (rc = upload(ctx, b->sr64, hsr)) || (rc = upload(ctx, b->user, b->user_host)) ||
       (rc = upload(ctx, b->devidx, b->dev_host)) ||
       (rc = upload(ctx, b->keys, hkeys)) || (rc = upload(ctx, b->blk_sys, hblk_sys)) ||
-      (rc = upload(ctx, b->blk_info, hblk_info)) || (rc = upload(ctx, b->items, hitems)) ||
+      (rc = upload(ctx, b->blk_info, hblk_info)) || (rc = upload(ctx, b->items, he64.born)) ||
+      (rc = upload(ctx, b->items_e, he64.pair)) || (rc = upload(ctx, b->tiles_e, he64.tiles)) ||
       (rc = upload(ctx, b->excl_ent, hent)) || (rc = upload(ctx, b->excl_rows, hrows)) ||
       (rc = upload(ctx, d_bidx, bidx)) || (rc = upload(ctx, d_bpar, bpar)) ||
       (rc = upload(ctx, d_aidx, aidx)) || (rc = upload(ctx, d_apar, apar)) ||
@@ -1143,20 +1159,28 @@ static cudaError_t enqueue_energy64(pb2_batch *b, cudaStream_t st) {
   ea.excl_ent = b->excl_ent;
   ea.excl_rows = b->excl_rows;
   ea.x = b->x; ea.y = b->y; ea.z = b->z;
-  ea.q = b->q64; ea.hs = b->hs64; ea.se = b->se64; ea.ro = b->ro64; ea.sr = b->sr64;
+  ea.q = b->charge; ea.hs = b->hs64; ea.se = b->se64; ea.ro = b->ro64; ea.sr = b->sr64;
   ea.radius = b->radius;
   ea.born64 = b->born64;
+  ea.iborn64 = b->iborn64;
   ea.born_acc = b->born_acc64;
   ea.energy = b->energy;
   ea.bbox = b->bbox;
   ea.blk_sys = b->blk_sys;
   ea.n_blocks = b->n_blocks;
   ea.sched = b->sched + kSchedE64;
+  ea.tiles = nullptr;
+  ea.n_tiles = 0;
   if (b->params.terms & PB2_USE_GB) {
     if ((e = launch_energy64(0, ea, b->grid_e64[0], st)) != cudaSuccess) return e;
     if ((e = launch_finalize64(ea, st)) != cudaSuccess) return e;
   }
   ea.sched = b->sched + kSchedE64 + 2;
+  ea.items = b->items_e;
+  ea.n_items = b->n_items_e;
+  ea.tiles = b->tiles_e;
+  ea.n_tiles = b->n_tiles_e;
+  if ((e = launch_energy64_tiles(ea, b->grid_tiles_e, st)) != cudaSuccess) return e;
   return launch_energy64(1, ea, b->grid_e64[1], st);
 }
 

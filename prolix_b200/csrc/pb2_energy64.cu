@@ -191,10 +191,13 @@ struct E64Masks {
   double cut2, gcut2, lj14, coul14;
   bool use_gb, use_lj, use_coul;
 };
+struct E64Sums {
+  double gb, coul, lj;
+};
 template <bool FULL>
 __device__ __forceinline__ void pair64(const E64Pair &I, double dx, double dy, double dz, double qj, double hsj,
                                        double sej, double Bj, double iBj, bool ok, bool ex, bool s14,
-                                       const E64Masks &M, double &e_gb, double &e_coul, double &e_lj) {
+                                       const E64Masks &M, E64Sums &E) {
   double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
   const double qq = I.q * qj;
   if (FULL || M.use_gb) {
@@ -204,7 +207,7 @@ __device__ __forceinline__ void pair64(const E64Pair &I, double dx, double dy, d
       qg = 0.0;
     }
     const double e = exp2neg_d(rg2 * (I.iB * iBj));
-    e_gb = fma(qg, rsqrt_d(fma(I.B * Bj, e, rg2)), e_gb);
+    E.gb = fma(qg, rsqrt_d(fma(I.B * Bj, e, rg2)), E.gb);
   }
   if (FULL || M.use_coul || M.use_lj) {
     double fc = 1.0, fl = 1.0;
@@ -218,29 +221,28 @@ __device__ __forceinline__ void pair64(const E64Pair &I, double dx, double dy, d
       }
     }
     const double inv_r = rsqrt_d(r2);
-    if (FULL || M.use_coul) e_coul = fma(FULL ? qq : qq * fc, inv_r, e_coul);
+    if (FULL || M.use_coul) E.coul = fma(FULL ? qq : qq * fc, inv_r, E.coul);
     if (FULL || M.use_lj) {
       const double t = (I.hs + hsj) * inv_r;
       const double t2 = t * t, s6 = t2 * t2 * t2;
       const double eps = I.se * sej;
-      e_lj = fma(FULL ? eps : eps * fl, fma(s6, s6, -s6), e_lj);
+      E.lj = fma(FULL ? eps : eps * fl, fma(s6, s6, -s6), E.lj);
     }
   }
 }
 
 template <bool FULL>
 __device__ __forceinline__ void pair64_tile(const E64Pair &I0, const E64Pair &I1, const E64Tile &T, int k0, int kn,
-                                            int lane, const E64Masks &M, double &e_gb, double &e_coul,
-                                            double &e_lj) {
+                                            int lane, const E64Masks &M, E64Sums &E0, E64Sums &E1) {
 #pragma unroll 1
   for (int k = k0; k < k0 + kn; ++k) {
     const int c = (lane + k) & 31;
     const double xj = T[0][c], yj = T[1][c], zj = T[2][c], qj = T[3][c], hsj = T[4][c], sej = T[5][c],
                  Bj = T[6][c], iBj = T[7][c];
     pair64<FULL>(I0, I0.x - xj, I0.y - yj, I0.z - zj, qj, hsj, sej, Bj, iBj, (M.V0 >> k) & 1u, (M.E0 >> k) & 1u,
-                 (M.S0 >> k) & 1u, M, e_gb, e_coul, e_lj);
+                 (M.S0 >> k) & 1u, M, E0);
     pair64<FULL>(I1, I1.x - xj, I1.y - yj, I1.z - zj, qj, hsj, sej, Bj, iBj, (M.V1 >> k) & 1u, (M.E1 >> k) & 1u,
-                 (M.S1 >> k) & 1u, M, e_gb, e_coul, e_lj);
+                 (M.S1 >> k) & 1u, M, E1);
   }
 }
 
@@ -258,18 +260,79 @@ __device__ __forceinline__ double e64_box_dist2(const float4 *bbox, int a, int b
 // sqrt(log2(e) / 4): exp(-r^2 / (4 B_i B_j)) = 2^-(r^2 iB_i iB_j)
 constexpr double kSqrtQuarterLog2eD = 0.60056120439322491;
 
-// The warp's energy sums of one item, added to its system's accumulators.
-__device__ __forceinline__ void flush_energy64(const Energy64Args &a, int sys, double e_gb, double e_coul,
-                                               double e_lj, int lane) {
-  e_gb = warp_sum_d(e_gb);
-  e_coul = warp_sum_d(e_coul);
-  e_lj = warp_sum_d(e_lj);
-  if (lane == 0) {
-    const SysInfo &S = a.sys[sys];
-    long long *e = a.energy + (size_t)sys * PB2_NTERMS;
-    atomic_add_fix(&e[PB2_TERM_GB], to_fix(2.0 * S.pref_d * e_gb, kEnergyScale));
-    atomic_add_fix(&e[PB2_TERM_COULOMB], to_fix(S.kcoul_d * e_coul, kEnergyScale));
-    atomic_add_fix(&e[PB2_TERM_LJ], to_fix(4.0 * e_lj, kEnergyScale));
+__device__ __forceinline__ E64Sums warp_sums(const E64Sums &E) {
+  return E64Sums{warp_sum_d(E.gb), warp_sum_d(E.coul), warp_sum_d(E.lj)};
+}
+
+// An i-block's sums of one item, added to its system's accumulators.
+__device__ __forceinline__ void add_energy64(const Energy64Args &a, int sys, const E64Sums &E) {
+  const SysInfo &S = a.sys[sys];
+  long long *e = a.energy + (size_t)sys * PB2_NTERMS;
+  atomic_add_fix(&e[PB2_TERM_GB], to_fix(2.0 * S.pref_d * E.gb, kEnergyScale));
+  atomic_add_fix(&e[PB2_TERM_COULOMB], to_fix(S.kcoul_d * E.coul, kEnergyScale));
+  atomic_add_fix(&e[PB2_TERM_LJ], to_fix(4.0 * E.lj, kEnergyScale));
+}
+
+__device__ __forceinline__ E64Pair load_pair64(const Energy64Args &a, int g, bool use_gb) {
+  E64Pair P{a.x[g], a.y[g], a.z[g], a.q[g], a.hs[g], a.se[g], 1.0, 1.0};
+  if (use_gb) {
+    P.B = a.born64[g];
+    P.iB = a.iborn64[g];
+  }
+  return P;
+}
+__device__ __forceinline__ void store_pair64(E64Tile &T, int lane, const E64Pair &J) {
+  T[0][lane] = J.x; T[1][lane] = J.y; T[2][lane] = J.z; T[3][lane] = J.q;
+  T[4][lane] = J.hs; T[5][lane] = J.se; T[6][lane] = J.B; T[7][lane] = J.iB;
+}
+
+// Pairs of lane i with j-lane c that exist: both atoms do, j > i on a diagonal.
+struct E64Valid {
+  uint32_t C0, C1;
+};
+__device__ __forceinline__ E64Valid valid64(int jb, int ib0, int n, bool iv0, bool iv1, int lane) {
+  const int nj = n - jb * 32;
+  const uint32_t jmask = nj >= 32 ? 0xffffffffu : ((1u << nj) - 1u);
+  const uint32_t diag_mask = lane == 31 ? 0u : (0xffffffffu << (lane + 1));
+  E64Valid v{iv0 ? jmask : 0u, iv1 ? jmask : 0u};
+  if (jb == ib0) {
+    v.C0 &= diag_mask;
+    v.C1 = 0u;
+  } else if (jb == ib0 + 1) {
+    v.C1 &= diag_mask;
+  }
+  return v;
+}
+
+// No pair of the energy pass beyond its root (0: unbounded).
+__device__ __forceinline__ double energy_reach2(const E64Masks &M) {
+  const bool direct = M.use_lj || M.use_coul;
+  if ((M.use_gb && !(M.gcut2 > 0.0)) || (direct && !(M.cut2 > 0.0))) return 0.0;
+  return fmax(M.use_gb ? M.gcut2 : 0.0, direct ? M.cut2 : 0.0);
+}
+
+// The exclusion rows of a tile's two i-blocks; ent: lanes 0-15 hold block
+// ib0's entries, 16-31 block ib0 + 1's.  True if the tile has any.
+__device__ __forceinline__ bool excl64(const Energy64Args &a, int2 ent, int jb, int lane, ExclRow &r0, ExclRow &r1) {
+  const unsigned hit = __ballot_sync(kFull, ent.x == jb);
+  const unsigned hit0 = hit & 0xffffu, hit1 = hit & 0xffff0000u;
+  r0 = r1 = ExclRow{0u, 0u};
+  if (hit0) r0 = a.excl_rows[__shfl_sync(kFull, ent.y, __ffs(hit0) - 1) + lane];
+  if (hit1) r1 = a.excl_rows[__shfl_sync(kFull, ent.y, __ffs(hit1) - 1) + lane];
+  return hit != 0u;
+}
+
+// Steps k0 .. k0 + kn - 1 of a tile's pair energies.
+__device__ __forceinline__ void pair64_steps(const E64Pair &P0, const E64Pair &P1, const E64Tile &T, int k0, int kn,
+                                             int lane, bool plain, const E64Valid &v, const ExclRow &r0,
+                                             const ExclRow &r1, E64Masks &M, E64Sums &E0, E64Sums &E1) {
+  if (plain) {
+    pair64_tile<true>(P0, P1, T, k0, kn, lane, M, E0, E1);
+  } else {
+    M.V0 = rotr_u32(v.C0, lane); M.V1 = rotr_u32(v.C1, lane);
+    M.E0 = rotr_u32(r0.excl, lane); M.E1 = rotr_u32(r1.excl, lane);
+    M.S0 = rotr_u32(r0.s14, lane); M.S1 = rotr_u32(r1.s14, lane);
+    pair64_tile<false>(P0, P1, T, k0, kn, lane, M, E0, E1);
   }
 }
 
@@ -289,7 +352,6 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
   M.use_lj = (a.terms & PB2_USE_LJ) != 0;
   M.use_coul = (a.terms & PB2_USE_COULOMB) != 0;
   const bool all_terms = M.use_gb && M.use_lj && M.use_coul;
-  const uint32_t diag_mask = lane == 31 ? 0u : (0xffffffffu << (lane + 1));
   const bool one_wave = a.n_items <= nwarps;  // no warp asks the counter for another item
   pdl_wait();
   pdl_trigger();
@@ -303,13 +365,7 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
     const double bcut2 = (double)S.born_cut2;
     // no pair of this pass beyond reach2 (0: unbounded); the boxes are of
     // the float32 positions, so the test leaves a margin for their rounding
-    double reach2 = bcut2;
-    if (PASS == 1) {
-      reach2 = 0.0;
-      const bool direct = M.use_lj || M.use_coul;
-      if ((!M.use_gb || M.gcut2 > 0.0) && (!direct || M.cut2 > 0.0))
-        reach2 = fmax(M.use_gb ? M.gcut2 : 0.0, direct ? M.cut2 : 0.0);
-    }
+    const double reach2 = PASS == 0 ? bcut2 : energy_reach2(M);
     const double skip2 = reach2 * 1.001 + 0.01;
     const bool cut = PASS == 0 ? bcut2 > 0.0 : (M.cut2 > 0.0 || M.gcut2 > 0.0);
     const int ib0 = item.iblk, ib1 = ib0 + 1;
@@ -325,20 +381,13 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
       A0 = load_born64(a, ig0, (double)S.ro_max);
       A1 = load_born64(a, ig1, (double)S.ro_max);
     } else {
-      auto load = [&](int g) {
-        E64Pair P{a.x[g], a.y[g], a.z[g], a.q[g], a.hs[g], a.se[g], 1.0, 1.0};
-        if (M.use_gb) {
-          P.B = a.born64[g];
-          P.iB = kSqrtQuarterLog2eD / P.B;
-        }
-        return P;
-      };
-      P0 = load(ig0);
-      P1 = load(ig1);
+      P0 = load_pair64(a, ig0, M.use_gb);
+      P1 = load_pair64(a, ig1, M.use_gb);
       if (lane < kExclPerBlock) ent = a.excl_ent[gib0 * kExclPerBlock + lane];
       else if (has1) ent = a.excl_ent[gib1 * kExclPerBlock + lane - kExclPerBlock];
     }
-    double acc0 = 0.0, acc1 = 0.0, e_gb = 0.0, e_coul = 0.0, e_lj = 0.0;
+    double acc0 = 0.0, acc1 = 0.0;
+    E64Sums E0{0.0, 0.0, 0.0}, E1{0.0, 0.0, 0.0};
     for (int jb = R.jb0; jb < R.jb1; ++jb) {
       const int gjb = S.blk_base + jb;
       double d2 = 0.0;
@@ -355,26 +404,13 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
         T[0][lane] = J.x; T[1][lane] = J.y; T[2][lane] = J.z;
         T[3][lane] = J.s2; T[4][lane] = J.s3; T[5][lane] = J.t2;
       } else {
-        T[0][lane] = a.x[jg]; T[1][lane] = a.y[jg]; T[2][lane] = a.z[jg];
-        T[3][lane] = a.q[jg]; T[4][lane] = a.hs[jg]; T[5][lane] = a.se[jg];
-        const double B = M.use_gb ? a.born64[jg] : 1.0;
-        T[6][lane] = B;
-        T[7][lane] = kSqrtQuarterLog2eD / B;
+        store_pair64(T, lane, load_pair64(a, jg, M.use_gb));
       }
       __syncwarp();
-      // pair validity of lane i with j-lane c: both exist, j > i on a diagonal
-      const int nj = n - jl0;
-      const uint32_t jmask = nj >= 32 ? 0xffffffffu : ((1u << nj) - 1u);
-      uint32_t C0 = iv0 ? jmask : 0u, C1 = iv1 ? jmask : 0u;
-      if (jb == ib0) {
-        C0 &= diag_mask;
-        C1 = 0u;
-      } else if (jb == ib1) {
-        C1 &= diag_mask;
-      }
-      const bool full = __all_sync(kFull, (C0 & C1) == 0xffffffffu) && !cut;
+      const E64Valid v = valid64(jb, ib0, n, iv0, iv1, lane);
+      const bool full = __all_sync(kFull, (v.C0 & v.C1) == 0xffffffffu) && !cut;
       if (PASS == 0) {
-        const E64Tests K{rotr_u32(C0, lane), rotr_u32(C1, lane), bcut2, ig0, ig1, off + jl0};
+        const E64Tests K{rotr_u32(v.C0, lane), rotr_u32(v.C1, lane), bcut2, ig0, ig1, off + jl0};
         const float *tier2 = S.tier2[0];
         const int k0 = R.k0, kn = R.kn;
         double accj = 0.0;
@@ -394,32 +430,21 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
         const int jc = jl0 + ((lane + k0 + kn) & 31);
         if (jc < n && accj != 0.0) atomic_add_fix(&a.born_acc[off + jc], to_fix(accj, kBornScale));
       } else {
-        uint32_t X0 = 0u, Y0 = 0u, X1 = 0u, Y1 = 0u;
-        const unsigned hit = __ballot_sync(kFull, ent.x == jb);
-        const unsigned hit0 = hit & 0xffffu, hit1 = hit & 0xffff0000u;
-        if (hit0) {
-          const ExclRow r = a.excl_rows[__shfl_sync(kFull, ent.y, __ffs(hit0) - 1) + lane];
-          X0 = r.excl; Y0 = r.s14;
-        }
-        if (hit1) {
-          const ExclRow r = a.excl_rows[__shfl_sync(kFull, ent.y, __ffs(hit1) - 1) + lane];
-          X1 = r.excl; Y1 = r.s14;
-        }
-        if (full && !hit && all_terms) {
-          pair64_tile<true>(P0, P1, T, R.k0, R.kn, lane, M, e_gb, e_coul, e_lj);
-        } else {
-          M.V0 = rotr_u32(C0, lane); M.V1 = rotr_u32(C1, lane);
-          M.E0 = rotr_u32(X0, lane); M.E1 = rotr_u32(X1, lane);
-          M.S0 = rotr_u32(Y0, lane); M.S1 = rotr_u32(Y1, lane);
-          pair64_tile<false>(P0, P1, T, R.k0, R.kn, lane, M, e_gb, e_coul, e_lj);
-        }
+        ExclRow r0, r1;
+        const bool hit = excl64(a, ent, jb, lane, r0, r1);
+        pair64_steps(P0, P1, T, R.k0, R.kn, lane, full && !hit && all_terms, v, r0, r1, M, E0, E1);
       }
     }
     if (PASS == 0) {
       if (iv0 && acc0 != 0.0) atomic_add_fix(&a.born_acc[ig0], to_fix(acc0, kBornScale));
       if (iv1 && acc1 != 0.0) atomic_add_fix(&a.born_acc[ig1], to_fix(acc1, kBornScale));
     } else {
-      flush_energy64(a, item.sys, e_gb, e_coul, e_lj, lane);
+      E0 = warp_sums(E0);
+      E1 = warp_sums(E1);
+      if (lane == 0) {
+        add_energy64(a, item.sys, E0);
+        add_energy64(a, item.sys, E1);
+      }
     }
     if (one_wave) break;
     int next = 0;
@@ -432,6 +457,81 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
     a.sched[0] = 0;
     a.sched[1] = 0;
   }
+}
+
+// Pair energies of the small systems (a.tiles): a thread block per tile, its
+// warps sharing the 32 steps.  The warps' sums meet in shared memory in warp
+// order and a tile's sums go to fixed point once per i-block: rounding each
+// warp's share by itself left the total of a 166-atom system 2e-9 off.
+constexpr int kTileWarps = 8;
+__global__ void __launch_bounds__(32 * kTileWarps) energy64_tile_kernel(const Energy64Args a) {
+  __shared__ E64Tile T;
+  __shared__ E64Sums s_e[2][kTileWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr int kn = 32 / kTileWarps;
+  E64Masks M;
+  M.use_gb = (a.terms & PB2_USE_GB) != 0;
+  M.use_lj = (a.terms & PB2_USE_LJ) != 0;
+  M.use_coul = (a.terms & PB2_USE_COULOMB) != 0;
+  pdl_wait();
+  pdl_trigger();
+  for (int u = (int)blockIdx.x; u < a.n_tiles; u += (int)gridDim.x) {
+    const TileItem item = a.tiles[u];
+    const SysInfo &S = a.sys[item.sys];
+    const int n = S.n, off = S.off, jb = item.jb0;
+    M.cut2 = (double)S.cutoff2; M.gcut2 = (double)S.gb_cutoff2;
+    M.lj14 = (double)S.lj14; M.coul14 = (double)S.coul14;
+    const int ib0 = item.iblk;
+    const bool has1 = ib0 + 1 < S.nblk;
+    const int gib0 = S.blk_base + ib0, gib1 = gib0 + (has1 ? 1 : 0);
+    const int il0 = ib0 * 32 + lane, il1 = il0 + 32, jl = jb * 32 + lane;
+    const bool iv0 = il0 < n, iv1 = il1 < n;
+    const double reach2 = energy_reach2(M);
+    if (reach2 > 0.0) {  // as energy64_kernel
+      double d2 = e64_box_dist2(a.bbox, gib0, S.blk_base + jb);
+      if (has1 && jb > ib0) d2 = fmin(d2, e64_box_dist2(a.bbox, gib1, S.blk_base + jb));
+      if (d2 >= reach2 * 1.001 + 0.01) continue;  // block-uniform
+    }
+    const E64Pair P0 = load_pair64(a, off + (iv0 ? il0 : n - 1), M.use_gb);
+    const E64Pair P1 = load_pair64(a, off + (iv1 ? il1 : n - 1), M.use_gb);
+    int2 ent = make_int2(-1, -1);
+    if (lane < kExclPerBlock) ent = a.excl_ent[gib0 * kExclPerBlock + lane];
+    else if (has1) ent = a.excl_ent[gib1 * kExclPerBlock + lane - kExclPerBlock];
+    ExclRow r0, r1;
+    const bool hit = excl64(a, ent, jb, lane, r0, r1);
+    const E64Valid v = valid64(jb, ib0, n, iv0, iv1, lane);
+    const bool plain = __all_sync(kFull, (v.C0 & v.C1) == 0xffffffffu) && !hit && M.use_gb && M.use_lj &&
+                       M.use_coul && !(M.cut2 > 0.0 || M.gcut2 > 0.0);
+    if (w == 0) store_pair64(T, lane, load_pair64(a, off + (jl < n ? jl : n - 1), M.use_gb));
+    __syncthreads();
+    E64Sums E0{0.0, 0.0, 0.0}, E1{0.0, 0.0, 0.0};
+    pair64_steps(P0, P1, T, w * kn, kn, lane, plain, v, r0, r1, M, E0, E1);
+    E0 = warp_sums(E0);
+    E1 = warp_sums(E1);
+    if (lane == 0) {
+      s_e[0][w] = E0;
+      s_e[1][w] = E1;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      E64Sums t = s_e[threadIdx.x][0];
+      for (int k = 1; k < kTileWarps; ++k) {
+        const E64Sums &v = s_e[threadIdx.x][k];
+        t.gb += v.gb; t.coul += v.coul; t.lj += v.lj;
+      }
+      add_energy64(a, item.sys, t);
+    }
+  }
+}
+
+cudaError_t launch_energy64_tiles(const Energy64Args &a, int grid, cudaStream_t st) {
+  if (a.n_tiles <= 0) return cudaSuccess;
+  return launch_after(energy64_tile_kernel, grid, 32 * kTileWarps, st, a);
+}
+int energy64_tile_occupancy() {
+  int blocks = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, energy64_tile_kernel, 32 * kTileWarps, 0);
+  return blocks > 0 ? blocks : 1;
 }
 
 // FP64 Born radii from the descreening sums (cleared for the next
@@ -461,6 +561,7 @@ __global__ void __launch_bounds__(128) finalize64_kernel(const Energy64Args a) {
       const double r_in = a.radius[i], q = a.q[i];
       const BornRadius R = born_radius(isum, r_in, S.clamp != 0);
       a.born64[i] = R.B;
+      a.iborn64[i] = kSqrtQuarterLog2eD / R.B;
       e_gb = to_fix(S.pref_d * q * q * R.inv_b, kEnergyScale);
       e_ace = to_fix(ace_energy(r_in, R.B), kEnergyScale);
     }

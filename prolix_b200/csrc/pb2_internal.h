@@ -74,8 +74,8 @@ struct pb2_batch {
   int32_t *blk_sys = nullptr;
   int32_t *sched = nullptr;  // per pass (pair passes, then the FP64 energy passes): (next item, finished warps)
   int n_blocks = 0;
-  double *q64 = nullptr, *hs64 = nullptr, *se64 = nullptr, *ro64 = nullptr, *sr64 = nullptr;
-  double *born64 = nullptr;
+  double *hs64 = nullptr, *se64 = nullptr, *ro64 = nullptr, *sr64 = nullptr;
+  double *born64 = nullptr, *iborn64 = nullptr;
   double *stage = nullptr;  // 3 x (n_total, 3) row-major staging for host transfers
   // atom order: the batch stores atom g where the caller's arrays hold atom
   // user[g] (both batch-wide indices; systems keep their ranges)
@@ -101,6 +101,10 @@ struct pb2_batch {
   int32_t *warn_counts = nullptr;
   TileItem *items = nullptr;   // items of the FP64 energy kernels, every system's
   int n_items = 0;
+  // the same for the pair energies: of the systems that are not small, and
+  // the small systems' tiles
+  TileItem *items_e = nullptr, *tiles_e = nullptr;
+  int n_items_e = 0, n_tiles_e = 0, grid_tiles_e = 1;
   int grid_e64[2] = {1, 1};    // their two passes' grids
   long long *born_acc64 = nullptr;  // their descreening sums
   TileItem *items2 = nullptr;  // pair kernels: the live items (those of systems not retired)

@@ -126,13 +126,15 @@ struct Energy64Args {
   const double *x, *y, *z;
   const double *q, *hs, *se, *ro, *sr;  // charge, sigma/2, sqrt(eps), rho~, scaled radius
   const double *radius;
-  double *born64;
+  double *born64, *iborn64;  // B, sqrt(log2(e) / 4) / B
   long long *born_acc;   // this path's own descreening sums; zero between evaluations
   long long *energy;
   const float4 *bbox;
   const int32_t *blk_sys;
   int32_t n_blocks;
   int32_t *sched;        // (items taken, finished warps); zero between launches
+  const TileItem *tiles; // pair energies of the small systems: their tiles
+  int32_t n_tiles;
 };
 
 // Neighbour-list control words (NlArgs::ctl)
@@ -266,6 +268,8 @@ int team_occupancy(int pass, int warps, bool cut);
 // The descreening (pass 0) and energy (pass 1) kernels, and between them the
 // FP64 Born radii with the per-atom energies.
 cudaError_t launch_energy64(int pass, const Energy64Args &a, int grid, cudaStream_t st);
+cudaError_t launch_energy64_tiles(const Energy64Args &a, int grid, cudaStream_t st);
+int energy64_tile_occupancy();
 cudaError_t launch_finalize64(const Energy64Args &a, cudaStream_t st);
 int energy64_occupancy(int pass);
 cudaError_t launch_born_finalize(const FinalizeArgs &a, cudaStream_t st);
