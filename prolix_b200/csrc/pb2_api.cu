@@ -225,6 +225,23 @@ static void spatial_order(const double *pos, int n, std::vector<int> &ord) {
   for (int a = 0; a < n; a += 32) std::sort(ord.begin() + a, ord.begin() + std::min(n, a + 32));
 }
 
+// Stable sort by cost, longest first (a counting sort: a large batch has
+// hundreds of thousands of items of a few costs).
+static void longest_first(std::vector<TileItem> &items) {
+  auto cost = [](const TileItem &t) {
+    const ItemRange r = item_range(t);
+    return (size_t)(r.jb1 - r.jb0) * r.kn;
+  };
+  size_t most = 0;
+  for (const TileItem &t : items) most = std::max(most, cost(t));
+  std::vector<size_t> at(most + 2, 0);  // at[c + 1]: items longer than most - c, then their next place
+  for (const TileItem &t : items) ++at[most - cost(t) + 1];
+  for (size_t c = 1; c < at.size(); ++c) at[c] += at[c - 1];
+  std::vector<TileItem> out(items.size());
+  for (const TileItem &t : items) out[at[most - cost(t)]++] = t;
+  items.swap(out);
+}
+
 // Work items of the two-i-block kernels: even i-blocks ib (with ib + 1)
 // against j-blocks [j0, j1), j0 >= ib, of at most seg tiles, longest first.
 // Where few items are shorter than seg by nature (long rows), a sixth of each
@@ -252,9 +269,7 @@ static std::vector<TileItem> build_items2(const std::vector<SysInfo> &sinfo, int
       }
     }
   }
-  std::stable_sort(items.begin(), items.end(), [](const TileItem &p, const TileItem &q) {
-    return (p.jb1 - p.jb0) > (q.jb1 - q.jb0);
-  });
+  longest_first(items);
   return items;
 }
 
@@ -284,12 +299,8 @@ static E64Items build_items_e64(const std::vector<SysInfo> &sinfo) {
         (parts > 1 ? out.tiles : out.pair).push_back(whole);
       }
   }
-  auto cost = [](const TileItem &t) {
-    const ItemRange r = item_range(t);
-    return (r.jb1 - r.jb0) * r.kn;
-  };
-  for (auto *v : {&out.born, &out.pair})
-    std::stable_sort(v->begin(), v->end(), [&](const TileItem &p, const TileItem &q) { return cost(p) > cost(q); });
+  longest_first(out.born);
+  longest_first(out.pair);
   return out;
 }
 
@@ -302,9 +313,7 @@ static std::vector<TileItem> build_items4(const std::vector<SysInfo> &sinfo, int
     for (int ib = 0; ib < nblk; ib += 4)
       for (int j0 = ib; j0 < nblk; j0 += seg) items.push_back(TileItem{s, ib, j0, std::min(j0 + seg, nblk)});
   }
-  std::stable_sort(items.begin(), items.end(), [](const TileItem &p, const TileItem &q) {
-    return (p.jb1 - p.jb0) > (q.jb1 - q.jb0);
-  });
+  longest_first(items);
   return items;
 }
 
@@ -1071,19 +1080,14 @@ static cudaError_t enqueue_pass(pb2_batch *b, int pass, const PairArgs &a, cudaS
 
 // Force kernels on the current posq; force accumulators must be zero (or
 // hold contributions to keep) and born_acc zero.  bonded_energy: also
-// accumulate the (FP64) bonded energies.  boxes_ready: the launch before
-// wrote the block boxes (and ran the pair list's displacement test).
-static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_energy,
-                                  bool boxes_ready = false) {
+// accumulate the (FP64) bonded energies.  The launch before (a step, a
+// minimiser's move or place_kernel) wrote the block boxes and ran the pair
+// list's displacement test.
+static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_energy) {
   cudaError_t e;
   Timer tm{b, st};
   PairArgs pa = pair_args(b);
   const bool gb = (b->params.terms & PB2_USE_GB) != 0;
-  if (!boxes_ready && (e = tm(kTimBbox, [&] {
-         return launch_bbox(b->sys, b->blk_sys, b->posq, b->bbox, b->n_blocks, st,
-                            b->pl_on ? b->pl_ref : nullptr, b->pl_on ? b->pl_ctl : nullptr);
-       })) != cudaSuccess)
-    return e;
   if (b->pl_on && (e = tm(kTimBbox, [&] { return launch_pl_update(pl_args(b), b->grid_pl, st); })) != cudaSuccess)
     return e;
   if (gb) {
@@ -1197,7 +1201,7 @@ static int enqueue_eval(pb2_batch *b, cudaStream_t st, bool energy) {
     CUDA_TRY(ctx, enqueue_energy64(b, b->side));
     CUDA_TRY(ctx, cudaEventRecord(b->ev_side[1], b->side));
   }
-  CUDA_TRY(ctx, enqueue_forces(b, st, energy, true));
+  CUDA_TRY(ctx, enqueue_forces(b, st, energy));
   if (energy) CUDA_TRY(ctx, cudaStreamWaitEvent(st, b->ev_side[1], 0));
   return PB2_OK;
 }
@@ -1349,7 +1353,7 @@ static int run_eager(pb2_batch *b, int n_steps, cudaStream_t st) {
   for (int t = 0; t < n_steps; ++t) {
     const IntArgs ia = int_args(b, b->key_parity, t > 0);
     CUDA_TRY(ctx, tm(kTimStep, [&] { return launch_step(ia, st); }));
-    CUDA_TRY(ctx, enqueue_forces(b, st, false, true));
+    CUDA_TRY(ctx, enqueue_forces(b, st, false));
     b->key_parity ^= 1;
   }
   const IntArgs fa = int_args(b, b->key_parity, 0);
@@ -1371,7 +1375,7 @@ static int get_graph(pb2_batch *b, int chunk, int parity, cudaGraphExec_t *out) 
   int p = parity;
   for (int t = 0; t < chunk && err == cudaSuccess; ++t) {
     err = launch_step(int_args(b, p, t > 0), cs);
-    if (err == cudaSuccess) err = enqueue_forces(b, cs, false, true);
+    if (err == cudaSuccess) err = enqueue_forces(b, cs, false);
     p ^= 1;
   }
   if (err == cudaSuccess) err = launch_finish(int_args(b, p, 0), cs);
@@ -1711,10 +1715,10 @@ static int min_graph(pb2_batch *b, int mode, int chunk, cudaGraphExec_t *out) {
   for (int t = 0; t < chunk && err == cudaSuccess; ++t) {
     if (mode == 0) {
       err = launch_min(kMinOpSd, ma, nullptr, cs);
-      if (err == cudaSuccess) err = enqueue_forces(b, cs, false, true);
+      if (err == cudaSuccess) err = enqueue_forces(b, cs, false);
     } else {
       err = launch_min(kMinOpFireMove, ma, nullptr, cs);
-      if (err == cudaSuccess) err = enqueue_forces(b, cs, false, true);
+      if (err == cudaSuccess) err = enqueue_forces(b, cs, false);
       if (err == cudaSuccess) err = launch_min(kMinOpFireClose, ma, nullptr, cs);
     }
   }

@@ -274,13 +274,9 @@ cudaError_t launch_finalize64(const Energy64Args &a, cudaStream_t st);
 int energy64_occupancy(int pass);
 cudaError_t launch_born_finalize(const FinalizeArgs &a, cudaStream_t st);
 int tile_kernel_occupancy(int pass, bool cut, int shape);
-int tile_kernel_warps(int pass, int shape);  // warps per block of a pair pass
-// Bounding boxes of every 32-atom block.  With pl_ref / pl_ctl set, also
-// flags the pair list for a rebuild (pl_ctl[PL_DIRTY]) when an atom moved
-// more than half the skin since the list was built.
+// Bounding boxes of every 32-atom block.
 cudaError_t launch_bbox(const SysInfo *sys, const int32_t *blk_sys, const float4 *posq, float4 *bbox,
-                        int n_blocks, cudaStream_t st, const float4 *pl_ref = nullptr,
-                        int32_t *pl_ctl = nullptr);
+                        int n_blocks, cudaStream_t st);
 // Rebuild the pair list when flagged (one launch; returns at once when clean).
 cudaError_t launch_pl_update(const PlArgs &a, int grid, cudaStream_t st);
 // The live work list: items of all[0, n_all) whose system is not retired,

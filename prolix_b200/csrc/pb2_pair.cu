@@ -78,9 +78,8 @@ struct PData {  // per-atom data a lane holds (its i atom, or the j atom passing
   float s2, s3;  // s^2, s^3 of the scaled radius (far-field series)
 };
 
-// 4 / log2(e), and sqrt(log2(e) / 4): the force pass stores 1/B pre-scaled by
+// sqrt(log2(e) / 4): the force pass stores 1/B pre-scaled by
 // sqrt(log2(e)/4) so that exp(-r^2 / (4 B_i B_j)) = exp2(-r^2 iB_i iB_j).
-constexpr float kInvQuarterLog2e = 2.7725887222397811f;
 constexpr float kSqrtQuarterLog2e = 0.60056120439322491f;
 constexpr float kSixthRoot2 = 1.12246204830937298f;  // 2^(1/6)
 constexpr float kSqrtHalf = 0.70710678118654752f;
@@ -1455,47 +1454,20 @@ __global__ void __launch_bounds__(THREADS, MINB) force4_kernel(const __grid_cons
   }
 }
 
-// Per-block bounding boxes of the float32 positions: one warp per block.
-__global__ void bbox_kernel(const SysInfo *sys, const int32_t *blk_sys, const float4 *posq,
-                            float4 *bbox, int n_blocks, const float4 *pl_ref, int32_t *pl_ctl) {
+// Per-block bounding boxes of the float32 positions, one warp per block (for
+// the neighbour-list build; steps and evaluations write theirs themselves).
+__global__ void bbox_kernel(const SysInfo *sys, const int32_t *blk_sys, const float4 *posq, float4 *bbox,
+                            int n_blocks) {
   const int lane = threadIdx.x & 31;
-  const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int nw = (int)((gridDim.x * blockDim.x) >> 5);
   pdl_wait();
-  pdl_trigger();
-  bool moved = false;  // this lane saw an atom beyond skin / 2 of the pair list's reference
-  for (int b = w; b < n_blocks; b += nw) {
+  for (int b = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); b < n_blocks; b += nw) {
     const SysInfo &S = sys[blk_sys[b]];
-    const int lb = b - S.blk_base;
-    const int l = lb * 32 + lane;
-    const int i = S.off + (l < S.n ? l : lb * 32);
-    const float4 p = posq[i];
-    if (pl_ref) {
-      const float4 r = pl_ref[i];
-      const float dx = p.x - r.x, dy = p.y - r.y, dz = p.z - r.z;
-      moved |= (double)fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > S.skin_half2;
-    }
-    float lo[3] = {p.x, p.y, p.z}, hi[3] = {p.x, p.y, p.z};
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        lo[c] = fminf(lo[c], __shfl_xor_sync(kFull, lo[c], o));
-        hi[c] = fmaxf(hi[c], __shfl_xor_sync(kFull, hi[c], o));
-      }
-    if (lane == 0) {
-      bbox[2 * b] = make_float4(lo[0], lo[1], lo[2], 0.f);
-      bbox[2 * b + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
-    }
+    const int l = (b - S.blk_base) * 32 + lane;
+    const bool valid = l < S.n;
+    block_box(bbox, b, lane, valid, valid ? posq[S.off + l] : make_float4(0.f, 0.f, 0.f, 0.f));
   }
-  if (pl_ctl && __any_sync(kFull, moved) && lane == 0) atomicOr(&pl_ctl[PL_DIRTY], 1);
 }
-
-// Born radii from the descreening sums, plus the per-atom GB self term
-// (q_i^2 / B_i, generalized_born.py:200-206, :410-413) and ACE
-// (:600-648), written as the initial value of dE/dB.  Clears the sums.
-// FP64: one evaluation per atom.
-
 
 // --------------------------------------------------------------- launchers
 
@@ -1590,10 +1562,9 @@ int team_occupancy(int pass, int warps, bool cut) {
 }
 
 cudaError_t launch_bbox(const SysInfo *sys, const int32_t *blk_sys, const float4 *posq, float4 *bbox,
-                        int n_blocks, cudaStream_t st, const float4 *pl_ref, int32_t *pl_ctl) {
+                        int n_blocks, cudaStream_t st) {
   if (n_blocks <= 0) return cudaSuccess;
-  const int grid = (n_blocks + 7) / 8;
-  return launch_after(bbox_kernel, grid, 256, st, sys, blk_sys, posq, bbox, n_blocks, pl_ref, pl_ctl);
+  return launch_after(bbox_kernel, (n_blocks + 7) / 8, 256, st, sys, blk_sys, posq, bbox, n_blocks);
 }
 
 cudaError_t launch_born_finalize(const FinalizeArgs &a, cudaStream_t st) {
@@ -1681,12 +1652,6 @@ int tile_shape(int pass, int shape, int *threads, int *min_blocks) {
   *threads = kShapes[pass][shape].threads;
   *min_blocks = kShapes[pass][shape].minb;
   return 0;
-}
-
-int tile_kernel_warps(int pass, int shape) {
-  int t = 256, m = 0;
-  tile_shape(pass, shape, &t, &m);
-  return t / 32;
 }
 
 int tile_kernel_occupancy(int pass, bool cut, int shape) {
