@@ -83,15 +83,21 @@ __device__ __forceinline__ double rsqrt_d(double a) {
   return mid_range(a) ? z : y;
 }
 
-// 2^-w for w >= 0: w = n + g with integer n, 2^-g by its polynomial, and n
-// off the exponent; zero from w = 1000 on (and for a NaN, which the caller's
-// r^2 carries on).
+// 2^-w: w = n + g with integer n, 2^-g by its polynomial, and n off the
+// exponent; zero from w = 1000 on.  SIGNED: w may be negative (one Born radius
+// of a pair is, where an atom's radius is below the dielectric offset), and
+// from -1000 down the answer is infinity.  A NaN takes any of these: the
+// caller's r^2 or Born radii carry it on.
+template <bool SIGNED>
 __device__ __forceinline__ double exp2neg_d(double w) {
   const double magic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer
   const double t = w + magic;
   const double p = exp2neg_poly(w - (t - magic));
   const double v = __hiloint2double(__double2hiint(p) - (__double2loint(t) << 20), __double2loint(p));
-  return (unsigned)__double2hiint(w) < 0x408f4000u ? v : 0.0;
+  const int hi = __double2hiint(w);
+  if (!SIGNED) return (unsigned)hi < 0x408f4000u ? v : 0.0;
+  if ((hi & 0x7fffffff) < 0x408f4000) return v;
+  return hi < 0 ? __hiloint2double(0x7ff00000, 0) : 0.0;
 }
 
 // The warp's closed-form queue: (i, j) batch atom indices.
@@ -185,7 +191,7 @@ __device__ __forceinline__ void born64_tile(const Energy64Args &a, const E64Born
 }
 
 // One tile of the energy pass.  FULL: every pair exists, no exclusion, no
-// cutoff, all three terms.
+// cutoff, all three terms.  SIGNED: a Born radius may be negative.
 struct E64Masks {
   uint32_t V0, V1, E0, E1, S0, S1;  // bit k: the pair of step k exists / excluded / 1-4
   double cut2, gcut2, lj14, coul14;
@@ -194,20 +200,20 @@ struct E64Masks {
 struct E64Sums {
   double gb, coul, lj;
 };
-template <bool FULL>
+template <bool FULL, bool SIGNED>
 __device__ __forceinline__ void pair64(const E64Pair &I, double dx, double dy, double dz, double qj, double hsj,
                                        double sej, double Bj, double iBj, bool ok, bool ex, bool s14,
                                        const E64Masks &M, E64Sums &E) {
   double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
   const double qq = I.q * qj;
   if (FULL || M.use_gb) {
-    double rg2 = r2 + 1e-12, qg = qq;
+    const double rg2 = r2 + 1e-12, e = exp2neg_d<SIGNED>(rg2 * (I.iB * iBj));
+    double f2 = fma(I.B * Bj, e, rg2), qg = qq;
     if (!FULL && !(ok && (M.gcut2 == 0.0 || r2 < M.gcut2))) {
-      rg2 = 1.0;
+      f2 = 1.0;  // a masked pair's own may have no root (a negative Born radius)
       qg = 0.0;
     }
-    const double e = exp2neg_d(rg2 * (I.iB * iBj));
-    E.gb = fma(qg, rsqrt_d(fma(I.B * Bj, e, rg2)), E.gb);
+    E.gb = fma(qg, rsqrt_d(f2), E.gb);
   }
   if (FULL || M.use_coul || M.use_lj) {
     double fc = 1.0, fl = 1.0;
@@ -231,7 +237,7 @@ __device__ __forceinline__ void pair64(const E64Pair &I, double dx, double dy, d
   }
 }
 
-template <bool FULL>
+template <bool FULL, bool SIGNED>
 __device__ __forceinline__ void pair64_tile(const E64Pair &I0, const E64Pair &I1, const E64Tile &T, int k0, int kn,
                                             int lane, const E64Masks &M, E64Sums &E0, E64Sums &E1) {
 #pragma unroll 1
@@ -239,9 +245,9 @@ __device__ __forceinline__ void pair64_tile(const E64Pair &I0, const E64Pair &I1
     const int c = (lane + k) & 31;
     const double xj = T[0][c], yj = T[1][c], zj = T[2][c], qj = T[3][c], hsj = T[4][c], sej = T[5][c],
                  Bj = T[6][c], iBj = T[7][c];
-    pair64<FULL>(I0, I0.x - xj, I0.y - yj, I0.z - zj, qj, hsj, sej, Bj, iBj, (M.V0 >> k) & 1u, (M.E0 >> k) & 1u,
+    pair64<FULL, SIGNED>(I0, I0.x - xj, I0.y - yj, I0.z - zj, qj, hsj, sej, Bj, iBj, (M.V0 >> k) & 1u, (M.E0 >> k) & 1u,
                  (M.S0 >> k) & 1u, M, E0);
-    pair64<FULL>(I1, I1.x - xj, I1.y - yj, I1.z - zj, qj, hsj, sej, Bj, iBj, (M.V1 >> k) & 1u, (M.E1 >> k) & 1u,
+    pair64<FULL, SIGNED>(I1, I1.x - xj, I1.y - yj, I1.z - zj, qj, hsj, sej, Bj, iBj, (M.V1 >> k) & 1u, (M.E1 >> k) & 1u,
                  (M.S1 >> k) & 1u, M, E1);
   }
 }
@@ -326,14 +332,17 @@ __device__ __forceinline__ bool excl64(const Energy64Args &a, int2 ent, int jb, 
 __device__ __forceinline__ void pair64_steps(const E64Pair &P0, const E64Pair &P1, const E64Tile &T, int k0, int kn,
                                              int lane, bool plain, const E64Valid &v, const ExclRow &r0,
                                              const ExclRow &r1, E64Masks &M, E64Sums &E0, E64Sums &E1) {
-  if (plain) {
-    pair64_tile<true>(P0, P1, T, k0, kn, lane, M, E0, E1);
-  } else {
-    M.V0 = rotr_u32(v.C0, lane); M.V1 = rotr_u32(v.C1, lane);
-    M.E0 = rotr_u32(r0.excl, lane); M.E1 = rotr_u32(r1.excl, lane);
-    M.S0 = rotr_u32(r0.s14, lane); M.S1 = rotr_u32(r1.s14, lane);
-    pair64_tile<false>(P0, P1, T, k0, kn, lane, M, E0, E1);
+  const int signs = __double2hiint(P0.iB) | __double2hiint(P1.iB) | __double2hiint(T[7][lane]);
+  const bool negative = __any_sync(kFull, signs < 0);
+  if (plain && !negative) {
+    pair64_tile<true, false>(P0, P1, T, k0, kn, lane, M, E0, E1);
+    return;
   }
+  M.V0 = rotr_u32(v.C0, lane); M.V1 = rotr_u32(v.C1, lane);
+  M.E0 = rotr_u32(r0.excl, lane); M.E1 = rotr_u32(r1.excl, lane);
+  M.S0 = rotr_u32(r0.s14, lane); M.S1 = rotr_u32(r1.s14, lane);
+  if (negative) pair64_tile<false, true>(P0, P1, T, k0, kn, lane, M, E0, E1);
+  else pair64_tile<false, false>(P0, P1, T, k0, kn, lane, M, E0, E1);
 }
 
 // PASS 0: descreening sums; PASS 1: pair energies.  The warps of one
