@@ -135,6 +135,10 @@ __device__ __forceinline__ E64Born load_born64(const Energy64Args &a, int g, dou
   const double s = a.sr[g], t = fmax(2.5 * s, s + ro_max);  // 2.5 = 1 / sqrt(kSeriesUNear)
   return E64Born{a.x[g], a.y[g], a.z[g], s * s, s * s * s, t * t};
 }
+// No position (a NaN): the closed form takes such a pair as nothing, the
+// series would carry it into the other atom's sum.
+__device__ __forceinline__ bool lost(const E64Born &A) { return isnan(A.x + A.y + A.z); }
+
 
 // One tile of the descreening pass, steps k0 .. k0 + kn - 1.  FAR: both
 // tiles in the series' domain; FULL: every pair exists and no cutoff.
@@ -395,6 +399,7 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
       if (lane < kExclPerBlock) ent = a.excl_ent[gib0 * kExclPerBlock + lane];
       else if (has1) ent = a.excl_ent[gib1 * kExclPerBlock + lane - kExclPerBlock];
     }
+    const bool lost_i = PASS == 0 && (lost(A0) || lost(A1));
     double acc0 = 0.0, acc1 = 0.0;
     E64Sums E0{0.0, 0.0, 0.0}, E1{0.0, 0.0, 0.0};
     for (int jb = R.jb0; jb < R.jb1; ++jb) {
@@ -407,11 +412,13 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
       }
       const int jl0 = jb * 32, jl = jl0 + lane;
       const int jg = off + (jl < n ? jl : n - 1);
+      bool series = true;  // every pair may take the series
       __syncwarp();  // every lane is done with the previous tile
       if (PASS == 0) {
         const E64Born J = load_born64(a, jg, (double)S.ro_max);
         T[0][lane] = J.x; T[1][lane] = J.y; T[2][lane] = J.z;
         T[3][lane] = J.s2; T[4][lane] = J.s3; T[5][lane] = J.t2;
+        series = !__any_sync(kFull, lost_i || lost(J));
       } else {
         store_pair64(T, lane, load_pair64(a, jg, M.use_gb));
       }
@@ -423,13 +430,13 @@ __global__ void __launch_bounds__(kE64Threads, PASS == 0 ? 4 : 3) energy64_kerne
         const float *tier2 = S.tier2[0];
         const int k0 = R.k0, kn = R.kn;
         double accj = 0.0;
-        if (full) {
+        if (full && series) {
           if (d2 >= tier2[0]) born64_tile<true, true, 0>(a, A0, A1, T, k0, kn, lane, K, acc0, acc1, accj, Q);
           else if (d2 >= tier2[1]) born64_tile<true, true, 1>(a, A0, A1, T, k0, kn, lane, K, acc0, acc1, accj, Q);
           else if (d2 >= tier2[2]) born64_tile<true, true, 2>(a, A0, A1, T, k0, kn, lane, K, acc0, acc1, accj, Q);
           else if (d2 >= S.far2) born64_tile<true, true, 3>(a, A0, A1, T, k0, kn, lane, K, acc0, acc1, accj, Q);
           else born64_tile<false, true, 3>(a, A0, A1, T, k0, kn, lane, K, acc0, acc1, accj, Q);
-        } else if (d2 >= S.far2) {
+        } else if (d2 >= S.far2 && series) {
           born64_tile<true, false, 3>(a, A0, A1, T, k0, kn, lane, K, acc0, acc1, accj, Q);
         } else {
           born64_tile<false, false, 3>(a, A0, A1, T, k0, kn, lane, K, acc0, acc1, accj, Q);

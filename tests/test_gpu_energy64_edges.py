@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from oracle import gbsa
-from prolix_b200 import _lib, engine
+from prolix_b200 import _lib, engine, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +43,23 @@ def test_a_pair_without_a_value_shows_in_the_energy(r, radius):
   with np.errstate(all="ignore"):
     assert not np.isfinite(gbsa.nonbonded(s, s["positions"])[0]["gb"])
   assert abs(_terms(s, terms=_lib.USE_GB)["gb"]) > 1e11
+
+
+def test_a_lost_atom_leaves_the_other_atoms_descreening_sums():
+  # one atom of an extended chain without a position (NaN): its pairs count
+  # as nothing in the descreening sums, near and far, so the nonpolar energy
+  # is that of the chain without the atom plus the atom's own, alone.  Each
+  # atom's energy is rounded to 2^-24; a Born sum to 2^-40 in each of at most
+  # 8 parts of each tile that touches the atom, and dACE/dI is below 20.
+  s = synth.make_chain(600, 5, compact=False, **synth.PHYSICAL_RANGES)
+  n, k = 600, 301
+  x = s["positions"].copy()
+  keep = np.arange(n) != k
+  born, _, _ = gbsa.born_radii(x[keep], s["radii"][keep], s["scaled_radii"][keep])
+  ref = gbsa.ace_energy(s["radii"][keep], born).sum()
+  ref += gbsa.ace_energy(s["radii"][k:k + 1], s["radii"][k:k + 1] - gbsa.DIELECTRIC_OFFSET)[0]
+  x[k, 1] = np.nan
+  with engine.Batch([s], terms=_lib.USE_GB) as b:
+    b.set_positions(x)
+    got = dict(zip(_lib.TERM_NAMES, b.energy_forces()[0][0]))["nonpolar"]
+  assert abs(got - ref) <= n * (2.0 ** -25 + 20.0 * 8 * 20 * 2.0 ** -41), (got, ref)
