@@ -160,9 +160,13 @@ __device__ __forceinline__ void born64_tile(const Energy64Args &a, const E64Born
     double r20 = fma(dx0, dx0, fma(dy0, dy0, fma(dz0, dz0, 1e-12)));
     double r21 = fma(dx1, dx1, fma(dy1, dy1, fma(dz1, dz1, 1e-12)));
     if (!FULL) {
-      const bool cut = M.bcut2 > 0.0;
-      if (!((M.V0 >> k) & 1u) || (cut && !(r20 - 1e-12 < M.bcut2))) r20 = kFarR2d;
-      if (!((M.V1 >> k) & 1u) || (cut && !(r21 - 1e-12 < M.bcut2))) r21 = kFarR2d;
+      bool in0 = (M.V0 >> k) & 1u, in1 = (M.V1 >> k) & 1u;
+      if (M.bcut2 > 0.0) {  // by r^2 itself: 1e-12 cannot be taken off again exactly
+        in0 = in0 && fma(dx0, dx0, fma(dy0, dy0, dz0 * dz0)) < M.bcut2;
+        in1 = in1 && fma(dx1, dx1, fma(dy1, dy1, dz1 * dz1)) < M.bcut2;
+      }
+      if (!in0) r20 = kFarR2d;
+      if (!in1) r21 = kFarR2d;
     }
     if (!FAR) {
       const double t2j = T[5][c];

@@ -63,3 +63,14 @@ def test_a_lost_atom_leaves_the_other_atoms_descreening_sums():
     b.set_positions(x)
     got = dict(zip(_lib.TERM_NAMES, b.energy_forces()[0][0]))["nonpolar"]
   assert abs(got - ref) <= n * (2.0 ** -25 + 20.0 * 8 * 20 * 2.0 ** -41), (got, ref)
+
+
+@pytest.mark.parametrize("cutoff", [4.0, 8.0, 9.0, 16.0])
+def test_a_pair_at_the_cutoff_is_outside_it(cutoff):
+  # r < cutoff counts: at the cutoff itself the energies are those of two
+  # atoms far apart, to the last bit
+  s = _two_atoms(cutoff, 1.5)
+  s["scaled_radii"][:] = 1.1
+  at = _terms(s, cutoff=cutoff)
+  assert at == _terms(dict(s, positions=s["positions"] * 3.0), cutoff=cutoff)
+  assert at != _terms(dict(s, positions=s["positions"] * 0.999), cutoff=cutoff)
