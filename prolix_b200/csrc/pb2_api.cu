@@ -273,6 +273,27 @@ static std::vector<TileItem> build_items2(const std::vector<SysInfo> &sinfo, int
   return items;
 }
 
+// Default length of those items: the longest (6, 4, 2 or 1 tiles, up to
+// `most`) that still gives every resident warp of the force pass a few items,
+// so a small batch spreads over the whole GPU.  us per step with 8, 6, 4, 2, 1:
+// a ragged batch of 256 systems, all pairs, 1308, 1308, 1325, 1346, 1398;
+// 20,000 atoms, all pairs, 817, 807, 806, 826, 891; with a direct cutoff of 9 A
+// beside GB over all pairs 885, 868, 867, 884, 953.  Where a reach drops tiles
+// whole, an item's cost varies and shorter ones even it out: without a pair
+// list at most two tiles (64 systems of 1,500 atoms at 9 A 420, 404, 386, 369,
+// 382; 20,000 atoms at 20 A 314, 289, 268, 284, 429), with one single tiles,
+// which come in no order (20,000 atoms at 20 A 260, 262, 232, 201, 193).
+static int default_segment(const std::vector<SysInfo> &sinfo, int most, int sm_count) {
+  for (int cand : {6, 4, 2}) {
+    if (cand > most) continue;
+    long long items = 0;
+    for (const SysInfo &S : sinfo)
+      for (int ib = 0; ib < S.nblk; ib += 2) items += (S.nblk - ib + cand - 1) / cand;
+    if (items >= 4LL * sm_count * 16) return cand;
+  }
+  return 1;
+}
+
 // Items of the FP64 energy kernels: pairs of i-blocks.  Each item's sums are
 // rounded to fixed point once, so how a system is cut depends on its own size
 // alone and its energies are the same in every batch.  A small system (up to
@@ -537,29 +558,6 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   if (!b) return fail(ctx, PB2_ENOMEM, "host allocation");
   b->ctx = ctx;
   b->params = *params;
-  if (b->params.tile_segment <= 0) {
-    // default work-item length: the longest (6, 4, 2 or 1 j-blocks) that still
-    // gives every resident warp of the force pass a few items, so a small
-    // batch spreads over the whole GPU; single tiles with a pair list, whose
-    // items come in no order.  us per step with 8, 6, 4, 2, 1: a ragged batch
-    // of 256 systems 1308, 1308, 1325, 1346, 1398; 20,000 atoms 817, 807, 806,
-    // 826, 891; the same at 20 A 264, 260, 232, 201, 191
-    const long long want = 4LL * ctx->sm_count * 16;
-    int seg = 1;
-    for (int cand : {6, 4, 2}) {
-      if (params->cutoff > 0.0) break;
-      long long items = 0;
-      for (int s = 0; s < n_systems; ++s) {
-        const int nb = (systems[s].n_atoms + 31) / 32;
-        for (int ib = 0; ib < nb; ib += 2) items += (nb - ib + cand - 1) / cand;
-      }
-      if (items >= want) {
-        seg = cand;
-        break;
-      }
-    }
-    b->params.tile_segment = seg;
-  }
   if (b->params.graph_chunk <= 0) b->params.graph_chunk = 50;
   b->n_sys = n_systems;
   const bool cutoff_mode = params->cutoff > 0.0;
@@ -883,25 +881,28 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   b->n_blocks = blocks_total;
   b->cut = cutoff_mode || gb_cut_mode || born_mode;
   {
-    // the pair list needs a finite reach for every pair term in use
+    // bounded: every pair term in use has a finite reach, as the pair list needs
     const uint32_t t = params->terms;
     const bool direct = (t & (PB2_USE_LJ | PB2_USE_COULOMB)) != 0, gbt = (t & PB2_USE_GB) != 0;
     double reach = 0.0;
-    bool finite = b->cut && params->skin >= 0.0 && params->pair_list >= 0;
+    bool bounded = b->cut && (direct || gbt);
     if (direct) {
-      finite = finite && cutoff_mode;
+      bounded = bounded && cutoff_mode;
       reach = std::max(reach, params->cutoff);
     }
     if (gbt) {
-      finite = finite && gb_cut_mode;
+      bounded = bounded && gb_cut_mode;
       reach = std::max(reach, std::max(gb_cut, born_cut));
     }
     // (it saves less than its update costs where no system has many blocks:
     // us per step with and without at 1,200 atoms, 20 A: 30.7, 29.0; 2,500,
-    // 9 A: 47.9, 51.2; 4,000, 12 A: 56.6, 59.7)
+    // 9 A: 47.9, 51.2; 4,000, 12 A: 56.6, 59.7; 64 systems of 1,500 atoms,
+    // 9 A: 382, 382)
     const bool many = std::any_of(sinfo.begin(), sinfo.end(), [](const SysInfo &S) { return S.nblk >= 64; });
-    b->pl_on = finite && (direct || gbt) && many;
+    b->pl_on = bounded && params->skin >= 0.0 && params->pair_list >= 0 && many;
     b->pl_reach2 = (float)((reach + params->skin) * (reach + params->skin));
+    if (b->params.tile_segment <= 0)
+      b->params.tile_segment = default_segment(sinfo, b->pl_on ? 1 : bounded ? 2 : 6, ctx->sm_count);
   }
   b->hs64 = D.alloc<double>(N);
   b->se64 = D.alloc<double>(N);
