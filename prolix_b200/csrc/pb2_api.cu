@@ -355,7 +355,7 @@ static void set_pair_grid(pb2_batch *b, int p) {
   const BondedArgs &ba = b->bonded;
   const int bonded = ba.n_bond + ba.n_angle + ba.n_tors + ba.n_cmap + ba.n_exc;
   const int chunks = (bonded + kBondedChunk - 1) / kBondedChunk;
-  const int units = b->n_items2 + (p == PASS_CHAIN ? chunks : p == PASS_BORN ? b->n_blocks : 0);
+  const int units = b->n_units2 + (p == PASS_CHAIN ? chunks : p == PASS_BORN ? b->n_blocks : 0);
   b->grid_pair[p] = std::max(1, std::min(cap, units));
 }
 
@@ -366,7 +366,7 @@ static void set_pair_grid(pb2_batch *b, int p) {
 // tiles 38.8 / 31.5 / 28.0; 1,500, 576 tiles 40.1 / 36.0 / 30.6; 1,800, 841
 // tiles 40.1 / 45.7 / 41.8.
 static void set_team(pb2_batch *b, int seg) {
-  const int n = b->n_items2;
+  const int n = b->n_units2;
   b->team = seg != 1 ? 0 : n <= 296 ? 8 : n <= 640 ? 4 : 0;
   if (!b->team) return;
   const BondedArgs &ba = b->bonded;
@@ -379,10 +379,16 @@ static void set_team(pb2_batch *b, int seg) {
 
 // (Re)build the pair kernels' two-i-block work list and their grids (one
 // resident wave each; warps take items dynamically).  The kernels read the
-// live list: the full one without the items of retired systems.
+// live list: the full one without the items of retired systems.  With a pair
+// list its items take their place, and these lists stay empty: at one tile
+// per item they would hold 48 B per tile beside the list's 36 (40,000 atoms
+// at 12 A: 1,335 B per atom with them, 866 without), and retiring a system
+// would compact them.
 static int setup_items2(pb2_batch *b, int seg) {
   pb2_ctx *ctx = b->ctx;
   std::vector<TileItem> items = build_items2(b->sys_host, seg);
+  b->n_units2 = (int)items.size();
+  if (b->pl_on) items = {};
   b->dev.release(b->items2);
   b->dev.release(b->items2_all);
   b->items2 = b->dev.alloc<TileItem>(std::max<size_t>(items.size(), 1));
@@ -400,7 +406,8 @@ static int setup_items2(pb2_batch *b, int seg) {
   }
   CUDA_TRY(ctx, launch_retire(-1, b->retired, b->items2_all, b->n_items2, b->items2, b->item_count, nullptr, nullptr));
   {
-    std::vector<TileItem> items4 = build_items4(b->sys_host, seg);
+    std::vector<TileItem> items4;
+    if (!b->pl_on) items4 = build_items4(b->sys_host, seg);
     b->dev.release(b->items4);
     b->dev.release(b->items4_all);
     b->items4 = b->dev.alloc<TileItem>(std::max<size_t>(items4.size(), 1));

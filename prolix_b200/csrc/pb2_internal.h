@@ -109,7 +109,8 @@ struct pb2_batch {
   long long *born_acc64 = nullptr;  // their descreening sums
   TileItem *items2 = nullptr;  // pair kernels: the live items (those of systems not retired)
   TileItem *items2_all = nullptr;  // every system's items over pairs of i-blocks
-  int n_items2 = 0;                // items in items2_all
+  int n_items2 = 0;                // items in items2_all (0 with a pair list)
+  int n_units2 = 0;                // items of all systems, with a pair list at most
   int32_t *item_count = nullptr;   // items in items2 (device)
   // the four-block force kernel's items (i-blocks ib % 4 == 0): all, live, counts
   TileItem *items4_all = nullptr, *items4 = nullptr;

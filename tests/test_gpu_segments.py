@@ -35,3 +35,25 @@ def test_single_tiles_with_a_pair_list():
   seg_off, f_off = _segment(systems, cutoff=9.0, pair_list=False)
   assert (seg, seg_off) == (1, 2)
   np.testing.assert_array_equal(f, f_off)
+
+
+def _device_bytes(systems, **kw):
+  """What the batch holds of the device's memory pool."""
+  from cuda.bindings import runtime as rt
+  attr = rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent
+  engine.Context.get(0)
+  pool = rt.cudaDeviceGetDefaultMemPool(0)[1]
+  before = int(rt.cudaMemPoolGetAttribute(pool, attr)[1])
+  with engine.Batch(systems, **kw):
+    return int(rt.cudaMemPoolGetAttribute(pool, attr)[1]) - before
+
+
+def test_the_pair_list_replaces_the_other_work_lists():
+  # 36 B per tile with it (two buffers of items and the j-blocks) against 48
+  # without at the same item length (two- and four-block items, all and live)
+  systems = [synth.make_chain(4000, 350, compact=True, **synth.PHYSICAL_RANGES)]
+  tiles = sum(125 - ib for ib in range(0, 125, 2))
+  listed = _device_bytes(systems, cutoff=12.0)
+  plain = _device_bytes(systems, cutoff=12.0, pair_list=False, tile_segment=1)
+  # the displacement reference and the rows: 16 B per atom and per pair of blocks
+  assert listed <= plain + 16 * 4000 + 16 * 63 + 8192, (listed, plain, tiles)
