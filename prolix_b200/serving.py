@@ -40,7 +40,36 @@ import numpy as np
 from . import engine, topology
 from ._lib import STATUS_FORCE_RANGE, STATUS_NONFINITE
 
-BYTES_PER_ATOM = 320  # device footprint of one atom in a batch (state, pair data, scratch)
+BYTES_PER_ATOM = 480  # device footprint of one atom in a batch (state, pair data, bonded terms, scratch)
+
+
+def system_bytes(n: int, cutoff: float = 0.0, cmap_points: int = 0) -> int:
+  """Device footprint of an ``n``-atom system in a cohort, at most: its atoms,
+  the work lists, which grow with its 32 x 32 tiles, and 128 B per grid point
+  of its CMAP tables."""
+  blocks = -(-n // 32)
+  tiles = sum(range(blocks, 0, -2))
+  # the FP64 energies' items: 16 B each, eight to one per tile (by the
+  # system's size), then two lists of several tiles per item
+  parts = 8 if blocks <= 28 else 4 if blocks <= 40 else 2 if blocks <= 57 else 1
+  span = 1 if blocks < 160 else 2 if blocks < 256 else 4 if blocks < 400 else 8
+  per_tile = 16 * (parts + 1) if parts > 1 else 32 / span
+  if cutoff > 0 and blocks >= 64:
+    per_tile += 36  # the pair list: two buffers of items, and the j-blocks
+  else:
+    # two- and four-block items, all and live, as long as the system alone
+    # (a larger cohort's are no shorter) would have them on 148 SMs
+    longest = 2 if cutoff > 0 else 6
+    items = {c: sum(-(-r // c) for r in range(blocks, 0, -2)) for c in (6, 4, 2) if c <= longest}
+    seg = next((c for c in items if items[c] >= 4 * 148 * 16), 1)
+    # (a sixth of a long row's tiles are two-block items of their own)
+    per_tile += 32 * min(1.0, 1 / seg + 1 / 6) + 16 / seg
+  return int(BYTES_PER_ATOM * n + per_tile * tiles + 128 * cmap_points)
+
+
+def _request_bytes(req, cutoff: float) -> int:
+  grids = req.system.get("cmap_energy_grids")
+  return system_bytes(len(req.system["charges"]), cutoff, 0 if grids is None else int(np.size(grids)))
 
 
 @dataclasses.dataclass
@@ -82,8 +111,9 @@ class _Slot:
 class _Cohort:
   """The systems admitted together: one device batch, one stream."""
 
-  def __init__(self, batch, slots, stream):
+  def __init__(self, batch, slots, stream, nbytes):
     self.batch = batch
+    self.bytes = nbytes   # device footprint
     self.slots = slots    # batch system index -> running slot, None once its request ended
     self.stream = stream  # a stream object with a .cuda_stream handle, or None
 
@@ -159,7 +189,7 @@ class Server:
     else:
       self._next_id = max(self._next_id, req.rid + 1)
     n = len(req.system["charges"])
-    if n * BYTES_PER_ATOM > self.hbm_budget or n > self.max_atoms:
+    if _request_bytes(req, self.cutoff) > self.hbm_budget or n > self.max_atoms:
       self.results[req.rid] = Result(req.rid, None, None, None, 0, req.arrival, float("nan"),
                                      self.now(), error="system larger than the server budget")
       return req.rid
@@ -181,9 +211,8 @@ class Server:
     return not self.queue and not self.cohorts
 
   # ------------------------------------------------------------------ internals
-  def _used(self):
-    atoms = sum(c.atoms() for c in self.cohorts)  # ended systems still hold their memory
-    return atoms, atoms * BYTES_PER_ATOM
+  def _used(self):  # ended systems still hold their memory
+    return sum(c.atoms() for c in self.cohorts), sum(c.bytes for c in self.cohorts)
 
   def _admit(self, now: float) -> list:
     """Take waiting requests while the budget allows (first come, first served)."""
@@ -197,12 +226,13 @@ class Server:
                                        now, error="cancelled")
         continue
       n = len(req.system["charges"])
-      if atoms + n > self.max_atoms or used + n * BYTES_PER_ATOM > self.hbm_budget:
+      need = _request_bytes(req, self.cutoff)
+      if atoms + n > self.max_atoms or used + need > self.hbm_budget:
         break  # first-come first-served: wait for room
       self.queue.popleft()
       admitted.append(req)
       atoms += n
-      used += n * BYTES_PER_ATOM
+      used += need
     return admitted
 
   def _fail(self, req, admitted, now, msg):
@@ -225,7 +255,8 @@ class Server:
         slots.append(None)
       else:
         slots.append(_Slot(r, 0, now))
-    cohort = _Cohort(batch, slots, self._streams() if self._streams else None)
+    cohort = _Cohort(batch, slots, self._streams() if self._streams else None,
+                     sum(_request_bytes(r, self.cutoff) for r in admitted))
     for b, s in enumerate(slots):
       if s is None and cohort.live():
         batch.retire(b, cohort.stream.cuda_stream if cohort.stream is not None else None)

@@ -4,7 +4,7 @@ every cutoff."""
 import numpy as np
 import pytest
 
-from prolix_b200 import engine, synth
+from prolix_b200 import engine, serving, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +57,23 @@ def test_the_pair_list_replaces_the_other_work_lists():
   plain = _device_bytes(systems, cutoff=12.0, pair_list=False, tile_segment=1)
   # the displacement reference and the rows: 16 B per atom and per pair of blocks
   assert listed <= plain + 16 * 4000 + 16 * 63 + 8192, (listed, plain, tiles)
+
+
+@pytest.mark.parametrize("cutoff", [0.0, 12.0])
+def test_the_server_counts_what_a_cohort_holds(cutoff):
+  # at most the server's figure, and no less than four fifths of it (a cohort
+  # of several systems has longer items than the figure takes for each alone)
+  for sizes in ((100,) * 40, (300, 900, 1900), (2500, 150), (10000,), (20000,)):
+    systems = []
+    for k, n in enumerate(sizes):
+      parts = [synth.make_chain(min(n, 2500), 360 + k, compact=True, **synth.PHYSICAL_RANGES) for _ in range(max(1, n // 2500))]
+      s = {f: np.concatenate([p[f] for p in parts]) for f in
+           ("charges", "sigmas", "epsilons", "radii", "scaled_radii", "masses", "bond_params", "angle_params",
+            "dihedral_params")}
+      for f in ("bonds", "angles", "dihedrals"):
+        s[f] = np.concatenate([p[f] + 2500 * j for j, p in enumerate(parts)])
+      s["positions"] = np.concatenate([p["positions"] + np.array([50.0 * j, 0.0, 0.0]) for j, p in enumerate(parts)])
+      systems.append(s)
+    held = _device_bytes(systems, cutoff=cutoff)
+    counted = sum(serving.system_bytes(n, cutoff) for n in sizes)
+    assert 0.8 * counted <= held <= counted, (sizes, held, counted)
