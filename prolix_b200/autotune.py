@@ -17,8 +17,9 @@ candidate (CUDA events on the launching stream; the fastest wins):
   against launches of their own.
 
 The best choice depends on the size mix of the batch; it is cached in JSON
-keyed by GPU name and a workload bucket (number of systems, total atoms,
-largest system, cutoff mode, each rounded to a power of two).  The batch's
+keyed by GPU name, a revision of the schedules to choose among, and a
+workload bucket (number of systems, total atoms, largest system, each rounded
+to a power of two, warps per tile at one tile per item, cutoff mode).  The batch's
 state is snapshotted before tuning and restored after, so tuning does not
 advance the simulation.
 
@@ -48,9 +49,24 @@ def _p2(x: float) -> int:
   return 1 << max(0, int(math.ceil(math.log2(max(1.0, float(x))))))
 
 
+# Of the schedules a choice is made among: a choice stored by a package with
+# other kernels (or none: before the kernels that share a tile, which items of
+# two tiles or more turn off) is not applied.
+SCHEDULE = 2
+# Tiles up to which a batch runs by thread blocks of 8 and of 4 warps per tile
+# (csrc/pb2_api.cu, set_team); its best segment is another on either side.
+TEAM_TILES = (296, 640)
+
+
+def team_warps(sizes) -> int:
+  """Warps that share a tile of a batch of these sizes at one tile per item."""
+  tiles = sum(sum(range(-(-int(n) // 32), 0, -2)) for n in sizes)
+  return 8 if tiles <= TEAM_TILES[0] else 4 if tiles <= TEAM_TILES[1] else 1
+
+
 def bucket_key(batch, gpu_name: str) -> str:
-  return "|".join([gpu_name, f"sys{_p2(batch.n_systems)}", f"atoms{_p2(batch.n_atoms)}",
-                   f"nmax{_p2(int(batch.sizes.max()))}",
+  return "|".join([gpu_name, f"v{SCHEDULE}", f"sys{_p2(batch.n_systems)}", f"atoms{_p2(batch.n_atoms)}",
+                   f"nmax{_p2(int(batch.sizes.max()))}", f"team{team_warps(batch.sizes)}",
                    "cut" if getattr(batch, "cutoff", 0.0) > 0 else "all"])
 
 
