@@ -220,12 +220,13 @@ int pb2_born_radii(pb2_batch *batch, double *born, void *stream);
 /* The same with DEVICE pointers on the batch's device: positions (may be
  * NULL: keep the current ones), energies (n_systems, PB2_NTERMS) and forces
  * (n_atoms_total, 3), row-major FP64, either may be NULL.  Asynchronous on
- * `stream`; allocates and synchronises nothing, so an XLA FFI handler (the
- * binding a prolix maintainer adds for make_energy_fn, system.py:29-271)
- * or a captured CUDA graph can call it.  The energies run on a stream of the
- * batch forked from `stream` and joined to it; from the third call on (outside
- * a capture) a small batch's launches are replayed as a CUDA graph,
- * instantiated then. */
+ * `stream`: synchronises nothing and allocates no buffers, so an XLA FFI
+ * handler (the binding a prolix maintainer adds for make_energy_fn,
+ * system.py:29-271) or a captured CUDA graph can call it.  The energies run on
+ * a stream of the batch forked from `stream` and joined to it.  Outside a
+ * capture of `stream`, a small batch's third call without energies and its
+ * third with them each instantiate a CUDA graph of the launches, which later
+ * calls replay; where that cannot be done, they launch. */
 int pb2_energy_forces_device(pb2_batch *batch, const double *positions, double *energies,
                              double *forces, void *stream);
 

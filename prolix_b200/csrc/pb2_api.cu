@@ -1218,29 +1218,30 @@ static int enqueue_eval(pb2_batch *b, cudaStream_t st, bool energy) {
 // host time is what a small system's evaluation waits for (166 atoms: 51 us
 // by launches, 37 as a graph; 2,500 atoms, 1,600 tiles: 92 and 100, since
 // consecutive graphs do not overlap).  Captured at the third evaluation (a
-// batch that is evaluated once or twice does not pay for it).
-static int eval_graph(pb2_batch *b, bool energy, cudaGraphExec_t *out) {
-  pb2_ctx *ctx = b->ctx;
-  if (!b->team) return PB2_OK;
-  *out = b->eval_graphs[energy];
-  if (*out || ++b->evals[energy] < 3) return PB2_OK;
+// batch that is evaluated once or twice does not pay for it), as work of this
+// thread alone: a capture in progress on another stream, of this thread or
+// another, neither forbids it nor is ended by it.  NULL: by launches, also
+// where no graph could be made.
+static cudaGraphExec_t eval_graph(pb2_batch *b, bool energy) {
+  if (!b->team) return nullptr;
+  cudaGraphExec_t &ex = b->eval_graphs[energy];
+  if (ex || ++b->evals[energy] < 3) return ex;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
   cudaStream_t cs = b->cap_stream;
-  CUDA_TRY(ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-  const int rc = enqueue_eval(b, cs, energy);
   cudaGraph_t g = nullptr;
-  const cudaError_t e = cudaStreamEndCapture(cs, &g);
-  if (rc || e != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
-    return rc ? rc : fail(ctx, PB2_ECUDA, std::string("graph capture failed: ") + cudaGetErrorString(e));
+  if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    const int rc = enqueue_eval(b, cs, energy);
+    if (cudaStreamEndCapture(cs, &g) == cudaSuccess && rc == PB2_OK && cudaGraphInstantiate(&ex, g, 0) != cudaSuccess)
+      ex = nullptr;
   }
-  const cudaError_t e2 = cudaGraphInstantiate(out, g, 0);
-  cudaGraphDestroy(g);
-  if (e2 != cudaSuccess) {
-    *out = nullptr;
-    return fail(ctx, PB2_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e2));
+  if (g) cudaGraphDestroy(g);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!ex) {
+    cudaGetLastError();   // the launches report their own
+    b->evals[energy] = 0;  // and the third call from here tries again
   }
-  b->eval_graphs[energy] = *out;
-  return PB2_OK;
+  return ex;
 }
 
 // Forces (and with energy set the FP64 energies) at the current positions,
@@ -1252,8 +1253,7 @@ static int fresh_forces(pb2_batch *b, cudaStream_t st, bool energy, const double
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (st) CUDA_TRY(ctx, cudaStreamIsCapturing(st, &cap));
   cudaGraphExec_t ex = nullptr;
-  if (cap == cudaStreamCaptureStatusNone && !b->profiling)
-    if (int rc = eval_graph(b, energy, &ex)) return rc;
+  if (cap == cudaStreamCaptureStatusNone && !b->profiling) ex = eval_graph(b, energy);
   if (ex) CUDA_TRY(ctx, cudaGraphLaunch(ex, st));
   else if (int rc = enqueue_eval(b, st, energy)) return rc;
   b->forces_valid = true;
