@@ -135,9 +135,13 @@ __device__ __forceinline__ E64Born load_born64(const Energy64Args &a, int g, dou
   const double s = a.sr[g], t = fmax(2.5 * s, s + ro_max);  // 2.5 = 1 / sqrt(kSeriesUNear)
   return E64Born{a.x[g], a.y[g], a.z[g], s * s, s * s * s, t * t};
 }
-// No position (a NaN): the closed form takes such a pair as nothing, the
-// series would carry it into the other atom's sum.
-__device__ __forceinline__ bool lost(const E64Born &A) { return isnan(A.x + A.y + A.z); }
+// No position (a NaN, or an infinity): the closed form takes a NaN's pairs as
+// nothing, the series would carry it into the other atom's sum.  By the
+// exponents, off the FP64 pipe.
+__device__ __forceinline__ bool lost(const E64Born &A) {
+  const int m = 0x7ff00000;
+  return (__double2hiint(A.x) & m) == m || (__double2hiint(A.y) & m) == m || (__double2hiint(A.z) & m) == m;
+}
 
 
 // One tile of the descreening pass, steps k0 .. k0 + kn - 1.  FAR: both
