@@ -364,10 +364,11 @@ static void set_pair_grid(pb2_batch *b, int p) {
 // lie where the step times cross (us per step, one system, all pairs; none /
 // 8 warps / 4 warps): 896 atoms, 210 tiles 36.9 / 22.5 / 24.9; 1,200, 380
 // tiles 38.8 / 31.5 / 28.0; 1,500, 576 tiles 40.1 / 36.0 / 30.6; 1,800, 841
-// tiles 40.1 / 45.7 / 41.8.
+// tiles 40.1 / 45.7 / 41.8.  Never with a pair list (its smallest batch, one
+// system of 64 blocks, has 1,056 tiles): the team kernels have no list.
 static void set_team(pb2_batch *b, int seg) {
   const int n = b->n_units2;
-  b->team = seg != 1 ? 0 : n <= 296 ? 8 : n <= 640 ? 4 : 0;
+  b->team = seg != 1 || b->pl_on ? 0 : n <= 296 ? 8 : n <= 640 ? 4 : 0;
   if (!b->team) return;
   const BondedArgs &ba = b->bonded;
   const int bonded = ba.n_bond + ba.n_angle + ba.n_tors + ba.n_cmap + ba.n_exc;
@@ -1117,7 +1118,7 @@ static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_ene
     // summed (profiling keeps the separate launch, to time it)
     const bool fuse_finalize = !b->profiling && (b->fuse & PB2_FUSE_FINALIZE);
     // teams for all three passes: no finalize launch (profiling keeps it)
-    if (b->team && !fuse_finalize && !b->profiling && (b->force_blocks == 2 || b->pl_on)) {
+    if (b->team && !fuse_finalize && !b->profiling && b->force_blocks == 2) {
       pa.heads = 1;
       pa.fin = fa;
     }
@@ -1132,7 +1133,11 @@ static cudaError_t enqueue_forces(pb2_batch *b, cudaStream_t st, bool bonded_ene
         (e = tm(kTimFinalize, [&] { return launch_born_finalize(fa, st); })) != cudaSuccess)
       return e;
   }
-  pa.early = gb;  // the descreening pass lies between the positions and what follows
+  // The descreening pass lies between the positions and what follows.  A team
+  // pass that is early, and a bonded launch, read positions before they wait
+  // for the launch before: whatever writes positions has to be two launches
+  // back or more.
+  pa.early = gb;
   pa.sched = b->sched + 2 * PASS_FORCE;
   if (b->force_blocks == 4 && !b->pl_on) {
     PairArgs p4 = pa;

@@ -1064,17 +1064,8 @@ __global__ void __launch_bounds__(32 * W) team_kernel(const __grid_constant__ Pa
       waited = true;
     }
   };
-  const bool plm = CUT && a.pl_ctl != nullptr;
   const TileItem *items = a.items;
-  int n_items = 0;
-  if (plm) {  // written by the list's update: with the descreening pass between, older than the launch before
-    if (!a.early) wait();
-    const int cur = a.pl_ctl[PL_CUR];
-    items = cur ? a.pl_items1 : a.pl_items0;
-    n_items = a.pl_ctl[PL_COUNT0 + cur];
-  } else {
-    n_items = *a.item_count;
-  }
+  const int n_items = *a.item_count;
   // units: W bonded chunks each (the longest), then the items
   const int n_bonded = PASS == PASS_CHAIN ? (a.n_bonded_chunks + W - 1) / W : 0;
   // a unit for every block: none asks the counter for another (a round trip
@@ -1104,8 +1095,7 @@ __global__ void __launch_bounds__(32 * W) team_kernel(const __grid_constant__ Pa
       PData I0, I1;
       load_par(a, ig0, S.ro_max, I0);
       load_par(a, ig1, S.ro_max, I1);
-      for (int tt = item.jb0; tt < item.jb1; ++tt) {
-        const int jb = plm ? a.pl_jlist[tt] : tt;
+      for (int jb = item.jb0; jb < item.jb1; ++jb) {
         const int jl0 = jb * 32, jl = jl0 + lane;
         const bool jvalid = jl < n;
         const int jg = off + (jvalid ? jl : n - 1);
