@@ -177,12 +177,15 @@ typedef struct pb2_run_params {
                               (compact 32-atom blocks, which the pair kernels' bounding-box
                               tests favour); 1: in input order.  Either way every array
                               crossing this interface is in input order. */
-  int32_t pair_list;    /* 0: automatic: when every pair term in use has a cutoff, the pair
-                           kernels work from a skin-buffered list of 32-atom block pairs
-                           within cutoff + skin, rebuilt on the device when an atom has
-                           moved more than skin/2 since the last build (jax_md's
-                           dr_threshold rule, batched_simulate.py:1600-1622); -1: off (every
-                           block pair, culled by bounding boxes at each step) */
+  int32_t pair_list;    /* 0: automatic: when every pair term in use has a cutoff and some
+                           system has 64 32-atom blocks or more (over 2,016 atoms; below,
+                           the list saves less than its update costs), the pair kernels
+                           work from a skin-buffered list of block pairs within
+                           cutoff + skin, rebuilt on the device when an atom has moved more
+                           than skin/2 since the last build (jax_md's dr_threshold rule,
+                           batched_simulate.py:1600-1622); -1: off (every block pair, culled
+                           by bounding boxes at each step).  The forces are the same bit for
+                           bit either way. */
 } pb2_run_params;
 
 typedef struct pb2_ctx pb2_ctx;
@@ -449,6 +452,12 @@ int pb2_retire_system(pb2_batch *batch, int32_t sys, void *stream);
  * is flagged with PB2_STATUS_WAIT_TIMEOUT while the other systems' results
  * stay exact.  Not for a batch with a pair list.  Waits for the device. */
 int pb2_test_hold_system(pb2_batch *batch, int32_t sys, int32_t hold);
+
+/* Test hook: how the batch runs as it is set up now: whether its cutoff runs
+ * use a pair list, warps that share a tile of the pair passes (0: each warp
+ * its own), and whether the last evaluation replayed a graph.  Any may be
+ * NULL. */
+int pb2_test_schedule(const pb2_batch *batch, int32_t *pair_list, int32_t *team, int32_t *replayed);
 
 /* Block shape of a pair pass (pass 0 descreening, 1 force, 2 chain rule,
  * 3 the force pass's four-block kernel): threads per block and the resident

@@ -1259,6 +1259,7 @@ static int fresh_forces(pb2_batch *b, cudaStream_t st, bool energy, const double
   if (st) CUDA_TRY(ctx, cudaStreamIsCapturing(st, &cap));
   cudaGraphExec_t ex = nullptr;
   if (cap == cudaStreamCaptureStatusNone && !b->profiling) ex = eval_graph(b, energy);
+  b->eval_replayed = ex != nullptr;
   if (ex) CUDA_TRY(ctx, cudaGraphLaunch(ex, st));
   else if (int rc = enqueue_eval(b, st, energy)) return rc;
   b->forces_valid = true;
@@ -2107,6 +2108,14 @@ extern "C" int pb2_test_hold_system(pb2_batch *b, int32_t sys, int32_t hold) {
   CUDA_TRY(ctx, cudaDeviceSynchronize());
   const int32_t v = b->sys_items_host[sys] + hold;
   CUDA_TRY(ctx, cudaMemcpy(b->sys_items + sys, &v, sizeof v, cudaMemcpyHostToDevice));
+  return PB2_OK;
+}
+
+extern "C" int pb2_test_schedule(const pb2_batch *b, int32_t *pair_list, int32_t *team, int32_t *replayed) {
+  if (!b) return PB2_EINVAL;
+  if (pair_list) *pair_list = b->pl_on;
+  if (team) *team = b->team;
+  if (replayed) *replayed = b->eval_replayed;
   return PB2_OK;
 }
 

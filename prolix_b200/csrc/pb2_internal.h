@@ -142,6 +142,7 @@ struct pb2_batch {
   // evaluations without and with energies: graph, and calls before it
   cudaGraphExec_t eval_graphs[2] = {nullptr, nullptr};
   int evals[2] = {0, 0};
+  bool eval_replayed = false;  // the last evaluation was a graph
   cudaStream_t side = nullptr;  // the FP64 energies of an evaluation, beside its forces
   cudaEvent_t ev_side[2] = {nullptr, nullptr};
   bool profiling = false;
