@@ -266,10 +266,11 @@ __device__ __forceinline__ ForceMasks force_masks(uint32_t V0, uint32_t V1, uint
 // (force_pair_factors: returns g, the force over the distance vector; hands h,
 // the numerator of dE/dB, to `on_h` where GB is in use), then the i-side sums
 // into ti and the j-side sums into tj (not rotated here).  Every force kernel
-// uses these functions, so their sums are the same bit for bit.  (h is handed
-// on inside the GB branch: a second branch on it after the factors costs a
-// pass without GB 3 %, 404 against 416 us per step for 256 ragged systems,
-// Lennard-Jones alone.)
+// uses these functions, so their sums are the same bit for bit.  LATE: the
+// sums of h after the factors, where they lengthen nothing; that takes a
+// second branch on GB, so only where GB is known to be in use.  us per step,
+// 256 ragged systems, Lennard-Jones alone: 416 late, 402 in the branch; 10,000
+// atoms at 20 A, all terms: 108.6 late, 110.4 in the branch.
 template <bool CUT, bool FULL, bool EXCL, class OnH>
 __device__ __forceinline__ float2 force_pair_factors(const FData2 &I, const JF2 &J, float2 dx, float2 dy, float2 dz,
                                                      ForceMasks &M, const TileConst &K, OnH on_h) {
@@ -333,16 +334,22 @@ __device__ __forceinline__ float2 force_pair_factors(const FData2 &I, const JF2 
   return g;
 }
 
-template <bool CUT, bool FULL, bool EXCL>
+template <bool CUT, bool FULL, bool EXCL, bool LATE>
 __device__ __forceinline__ void force_pair_step(const FData2 &I, const JF2 &J, Acc2F &ti, Acc &tj, ForceMasks &M,
                                                 const TileConst &K) {
   const float2 dx = __fadd2_rn(I.x, J.mx);
   const float2 dy = __fadd2_rn(I.y, J.my);
   const float2 dz = __fadd2_rn(I.z, J.mz);
-  const float2 g = force_pair_factors<CUT, FULL, EXCL>(I, J, dx, dy, dz, M, K, [&](float2 h) {
+  float2 late = make_float2(0.f, 0.f);
+  auto sum_h = [&](float2 h) {
     ti.a3 = __fadd2_rn(ti.a3, h);
     tj.a3 = tj.a3 + h.x + h.y;
+  };
+  const float2 g = force_pair_factors<CUT, FULL, EXCL>(I, J, dx, dy, dz, M, K, [&](float2 h) {
+    if (LATE) late = h;
+    else sum_h(h);
   });
+  if (LATE) sum_h(late);
   ti.a0 = __ffma2_rn(g, dx, ti.a0);
   ti.a1 = __ffma2_rn(g, dy, ti.a1);
   ti.a2 = __ffma2_rn(g, dz, ti.a2);
@@ -356,7 +363,7 @@ __device__ __forceinline__ void rotate_force(Acc &tj, int src, const TileConst &
   rotate_force_rest(tj, src, K);
 }
 
-template <bool CUT, bool FULL, bool EXCL>
+template <bool CUT, bool FULL, bool EXCL, bool ALL>
 __device__ __forceinline__ void run_force_tile2(const FData2 &I, const JTile &jt, Acc2F &ti, Acc &tj, uint32_t V0,
                                                 uint32_t V1, uint32_t E0, uint32_t E1, uint32_t S0,
                                                 uint32_t S1, const TileConst &K) {
@@ -365,7 +372,7 @@ __device__ __forceinline__ void run_force_tile2(const FData2 &I, const JTile &jt
 #pragma unroll kUnroll
   for (int k = 0; k < 32; ++k) {
     const JF2 J = load_jf(jt, K.lane + k);  // lane l meets j-lane (l + k) mod 32
-    force_pair_step<CUT, FULL, EXCL>(I, J, ti, tj, M, K);
+    force_pair_step<CUT, FULL, EXCL, ALL>(I, J, ti, tj, M, K);
     rotate_force(tj, K.src, K);
   }
 }
@@ -373,15 +380,15 @@ __device__ __forceinline__ void run_force_tile2(const FData2 &I, const JTile &jt
 // Four i-blocks: two packed pairs share each step's j atom (one set of
 // shared-memory loads for four pairs); each pair keeps its own j-side sums,
 // so the sums are those of two two-block tiles.
-template <bool CUT, bool FULL, bool EXCL>
+template <bool CUT, bool FULL, bool EXCL, bool ALL>
 __device__ __forceinline__ void run_force_tile4(const FData2 &Ia, const FData2 &Ib, const JTile &jt, Acc2F &ta,
                                                 Acc2F &tb, Acc &tja, Acc &tjb, ForceMasks Ma, ForceMasks Mb,
                                                 const TileConst &K) {
 #pragma unroll 1
   for (int k = 0; k < 32; ++k) {
     const JF2 J = load_jf(jt, K.lane + k);
-    force_pair_step<CUT, FULL, EXCL>(Ia, J, ta, tja, Ma, K);
-    force_pair_step<CUT, FULL, EXCL>(Ib, J, tb, tjb, Mb, K);
+    force_pair_step<CUT, FULL, EXCL, ALL>(Ia, J, ta, tja, Ma, K);
+    force_pair_step<CUT, FULL, EXCL, ALL>(Ib, J, tb, tjb, Mb, K);
     rotate_force(tja, K.src, K);
     rotate_force(tjb, K.src, K);
   }
@@ -848,9 +855,9 @@ __global__ void __launch_bounds__(THREADS, MINB)
           E1 = rotr32(r.excl, lane); S1 = rotr32(r.s14, lane);
         }
         Acc2F tf = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-        if (hit) run_force_tile2<CUT, false, true>(IF, jt, tf, tj, V0, V1, E0, E1, S0, S1, K);
-        else if (!full) run_force_tile2<CUT, false, false>(IF, jt, tf, tj, V0, V1, E0, E1, S0, S1, K);
-        else run_force_tile2<CUT, true, false>(IF, jt, tf, tj, V0, V1, E0, E1, S0, S1, K);
+        if (hit) run_force_tile2<CUT, false, true, ALL>(IF, jt, tf, tj, V0, V1, E0, E1, S0, S1, K);
+        else if (!full) run_force_tile2<CUT, false, false, ALL>(IF, jt, tf, tj, V0, V1, E0, E1, S0, S1, K);
+        else run_force_tile2<CUT, true, false, ALL>(IF, jt, tf, tj, V0, V1, E0, E1, S0, S1, K);
         t0.a0 = tf.a0.x; t0.a1 = tf.a1.x; t0.a2 = tf.a2.x; t0.a3 = tf.a3.x;
         t1.a0 = tf.a0.y; t1.a1 = tf.a1.y; t1.a2 = tf.a2.y; t1.a3 = tf.a3.y;
       } else {
@@ -1405,9 +1412,9 @@ __global__ void __launch_bounds__(THREADS, MINB) force4_kernel(const __grid_cons
       for (int h = 0; h < 2; ++h)
         tf[h] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       Acc tja = {0.f, 0.f, 0.f, 0.f}, tjb = {0.f, 0.f, 0.f, 0.f};
-      if (any_hit) run_force_tile4<CUT, false, true>(IF[0], IF[1], jt, tf[0], tf[1], tja, tjb, Ma, Mb, K);
-      else if (!full) run_force_tile4<CUT, false, false>(IF[0], IF[1], jt, tf[0], tf[1], tja, tjb, Ma, Mb, K);
-      else run_force_tile4<CUT, true, false>(IF[0], IF[1], jt, tf[0], tf[1], tja, tjb, Ma, Mb, K);
+      if (any_hit) run_force_tile4<CUT, false, true, ALL>(IF[0], IF[1], jt, tf[0], tf[1], tja, tjb, Ma, Mb, K);
+      else if (!full) run_force_tile4<CUT, false, false, ALL>(IF[0], IF[1], jt, tf[0], tf[1], tja, tjb, Ma, Mb, K);
+      else run_force_tile4<CUT, true, false, ALL>(IF[0], IF[1], jt, tf[0], tf[1], tja, tjb, Ma, Mb, K);
 
       // j partials are back in their home lanes: both pairs' sums, added in
       // fixed point, in one atomic per component
