@@ -273,6 +273,16 @@ static std::vector<TileItem> build_items2(const std::vector<SysInfo> &sinfo, int
   return items;
 }
 
+// Items of `seg` tiles over all rows, tiles(s, ib) in the row of system s that
+// begins at i-block ib.
+template <class F>
+static long long count_items(const std::vector<SysInfo> &sinfo, int seg, F &&tiles) {
+  long long items = 0;
+  for (int s = 0; s < (int)sinfo.size(); ++s)
+    for (int ib = 0; ib < sinfo[s].nblk; ib += 2) items += (tiles(s, ib) + seg - 1) / seg;
+  return items;
+}
+
 // Default length of those items: the longest (6, 4, 2 or 1 tiles, up to
 // `most`) that still gives every resident warp of the force pass a few items,
 // so a small batch spreads over the whole GPU.  us per step with 8, 6, 4, 2, 1:
@@ -281,16 +291,52 @@ static std::vector<TileItem> build_items2(const std::vector<SysInfo> &sinfo, int
 // beside GB over all pairs 885, 868, 867, 884, 953.  Where a reach drops tiles
 // whole, an item's cost varies and shorter ones even it out: without a pair
 // list at most two tiles (64 systems of 1,500 atoms at 9 A 420, 404, 386, 369,
-// 382; 20,000 atoms at 20 A 314, 289, 268, 284, 429), with one single tiles,
-// which come in no order (20,000 atoms at 20 A 260, 262, 232, 201, 193).
+// 382; 20,000 atoms at 20 A 314, 289, 268, 284, 429).
 static int default_segment(const std::vector<SysInfo> &sinfo, int most, int sm_count) {
-  for (int cand : {6, 4, 2}) {
-    if (cand > most) continue;
-    long long items = 0;
-    for (const SysInfo &S : sinfo)
-      for (int ib = 0; ib < S.nblk; ib += 2) items += (S.nblk - ib + cand - 1) / cand;
-    if (items >= 4LL * sm_count * 16) return cand;
+  for (int cand : {6, 4, 2})
+    if (cand <= most && count_items(sinfo, cand, [&](int s, int ib) { return sinfo[s].nblk - ib; }) >= 4LL * sm_count * 16)
+      return cand;
+  return 1;
+}
+
+// The same with a pair list, whose items come in no order: the longest (4, 2
+// or 1 tiles) that gives every resident warp eight items of the tiles within
+// reach of the initial positions.  us per step with 4, 2, 1 and the items of
+// two tiles: 20,000 atoms at 20 A (7,800 items) 232, 201, 193; 40,000 at 20 A
+// (16,900) 389, 367, 365; 32 systems of 2,500 atoms at 12 A (18,900) 451, 428,
+// 432; 128 ragged systems at 12 A (22,200) 526, 507, 519; 256 of them at 12 A
+// (53,900, of four tiles 28,100) 1138, 1144, 1188, at 20 A 1410, 1424, 1482.
+static int listed_segment(const std::vector<SysInfo> &sinfo, const std::vector<float4> &posq, float reach2,
+                          int sm_count) {
+  std::vector<std::vector<int>> live(sinfo.size());
+  std::vector<float> box[6];  // block boxes: low x, y, z, high x, y, z
+  for (int s = 0; s < (int)sinfo.size(); ++s) {
+    const SysInfo &S = sinfo[s];
+    for (int c = 0; c < 6; ++c) box[c].assign(S.nblk + 1, c < 3 ? INFINITY : -INFINITY);
+    for (int l = 0; l < S.n; ++l) {
+      const float4 p = posq[S.off + l];
+      const float x[3] = {p.x, p.y, p.z};
+      for (int c = 0; c < 3; ++c) {
+        box[c][l / 32] = std::min(box[c][l / 32], x[c]);
+        box[3 + c][l / 32] = std::max(box[3 + c][l / 32], x[c]);
+      }
+    }
+    const float *lx = box[0].data(), *ly = box[1].data(), *lz = box[2].data();
+    const float *hx = box[3].data(), *hy = box[4].data(), *hz = box[5].data();
+    auto dist2 = [&](int a, int b) {
+      const float dx = std::max(0.f, std::max(lx[a] - hx[b], lx[b] - hx[a]));
+      const float dy = std::max(0.f, std::max(ly[a] - hy[b], ly[b] - hy[a]));
+      const float dz = std::max(0.f, std::max(lz[a] - hz[b], lz[b] - hz[a]));
+      return dx * dx + dy * dy + dz * dz;
+    };
+    for (int ib = 0; ib < S.nblk; ib += 2) {  // (block nblk is an empty box, out of every reach)
+      int n = 1;
+      for (int jb = ib + 1; jb < S.nblk; ++jb) n += std::min(dist2(ib, jb), dist2(ib + 1, jb)) < reach2;
+      live[s].push_back(n);
+    }
   }
+  for (int cand : {4, 2})
+    if (count_items(sinfo, cand, [&](int s, int ib) { return live[s][ib / 2]; }) >= 8LL * sm_count * 16) return cand;
   return 1;
 }
 
@@ -387,9 +433,10 @@ static void set_team(pb2_batch *b, int seg) {
 // would compact them.
 static int setup_items2(pb2_batch *b, int seg) {
   pb2_ctx *ctx = b->ctx;
-  std::vector<TileItem> items = build_items2(b->sys_host, seg);
-  b->n_units2 = (int)items.size();
-  if (b->pl_on) items = {};
+  std::vector<TileItem> items;
+  if (!b->pl_on) items = build_items2(b->sys_host, seg);
+  b->n_units2 = b->pl_on ? (int)count_items(b->sys_host, seg, [&](int s, int ib) { return b->sys_host[s].nblk - ib; })
+                         : (int)items.size();
   b->dev.release(b->items2);
   b->dev.release(b->items2_all);
   b->items2 = b->dev.alloc<TileItem>(std::max<size_t>(items.size(), 1));
@@ -910,7 +957,8 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
     b->pl_on = bounded && params->skin >= 0.0 && params->pair_list >= 0 && many;
     b->pl_reach2 = (float)((reach + params->skin) * (reach + params->skin));
     if (b->params.tile_segment <= 0)
-      b->params.tile_segment = default_segment(sinfo, b->pl_on ? 1 : bounded ? 2 : 6, ctx->sm_count);
+      b->params.tile_segment = b->pl_on ? listed_segment(sinfo, hposq, b->pl_reach2, ctx->sm_count)
+                                        : default_segment(sinfo, bounded ? 2 : 6, ctx->sm_count);
   }
   b->hs64 = D.alloc<double>(N);
   b->se64 = D.alloc<double>(N);

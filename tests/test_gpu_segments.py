@@ -77,3 +77,13 @@ def test_the_server_counts_what_a_cohort_holds(cutoff):
     held = _device_bytes(systems, cutoff=cutoff)
     counted = sum(serving.system_bytes(n, cutoff) for n in sizes)
     assert 0.8 * counted <= held <= counted, (sizes, held, counted)
+
+
+def test_item_length_with_a_pair_list_follows_the_tiles_within_reach():
+  # 24 systems of 2,500 atoms at 40 A list nearly all of their 38,400 tiles:
+  # two per item; at 6 A a third of them: one
+  systems = [synth.make_chain(2500, 340, compact=True, **synth.PHYSICAL_RANGES)] * 24
+  wide, f = _segment(systems, cutoff=40.0)
+  narrow, _ = _segment(systems, cutoff=6.0)
+  assert (wide, narrow) == (2, 1)
+  np.testing.assert_array_equal(f, _segment(systems, cutoff=40.0, pair_list=False)[1])
