@@ -1692,6 +1692,8 @@ static MinArgs min_args(pb2_batch *b) {
   a.par = b->m_par;
   a.n_total = b->n_total;
   a.n_sys = b->n_sys;
+  a.blk_info = b->blk_info;
+  a.n_blocks = b->n_blocks;
   a.chunks = b->m_chunks;
   a.chunk0 = b->m_chunk0;
   a.n_chunks = b->m_n_chunks;

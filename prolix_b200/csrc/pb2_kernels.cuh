@@ -226,7 +226,9 @@ struct MinArgs {
   uint32_t *status;
   const double *par;
   int32_t n_total, n_sys;
-  // thread blocks of the SD and FIRE kernels: (system, its first 32-atom
+  const int4 *blk_info;  // per 32-atom block: system, first atom, atoms
+  int32_t n_blocks;
+  // thread blocks of the FIRE kernels: (system, its first 32-atom
   // block) of each chunk, a system's first chunk, and their partial sums
   const int2 *chunks;
   const int32_t *chunk0;  // (n_sys + 1)
