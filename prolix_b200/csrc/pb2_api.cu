@@ -1004,10 +1004,7 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   double *d_ccoef = D.alloc<double>(ccoef.size());
   int32_t *d_cgrid = D.alloc<int32_t>(cgrid.size());
   int64_t *d_cmoff = D.alloc<int64_t>(cmoff.size());
-  for (void *p : D.ptrs)
-    if (!p) return fail(ctx, PB2_ENOMEM, "device allocation failed");
-  if (!d_cmoff || !d_cgrid || !d_ccoef || !d_cidx || !b->excl_rows)
-    return fail(ctx, PB2_ENOMEM, "device allocation failed");
+  if (D.failed) return fail(ctx, PB2_ENOMEM, "device allocation failed");
 
   int rc;
   if ((rc = upload(ctx, b->sys, sinfo)) || (rc = upload(ctx, b->atom_sys, hsys)) ||

@@ -31,6 +31,7 @@ constexpr int kTimBorn = 0, kTimFinalize = 1, kTimForce = 2, kTimChain = 3, kTim
 // ordered on the default stream after the owner has synchronised the device.
 struct Dev {
   std::vector<void *> ptrs;
+  bool failed = false;  // an allocation has failed
   ~Dev() {
     for (void *p : ptrs)
       if (p) cudaFreeAsync(p, 0);
@@ -39,9 +40,13 @@ struct Dev {
   T *alloc(size_t n) {
     void *p = nullptr;
     if (n == 0) n = 1;
-    if (cudaMallocAsync(&p, n * sizeof(T), 0) != cudaSuccess) return nullptr;
+    if (cudaMallocAsync(&p, n * sizeof(T), 0) != cudaSuccess) {
+      failed = true;
+      return nullptr;
+    }
     if (cudaStreamSynchronize(0) != cudaSuccess) {
       cudaFreeAsync(p, 0);
+      failed = true;
       return nullptr;
     }
     ptrs.push_back(p);
