@@ -174,9 +174,6 @@ static int forces_not_from_step(pb2_batch *b, cudaStream_t st) {
 
 IntArgs int_args_for_nl(pb2_batch *b) { return int_args(b, b->key_parity, 0); }
 
-// Tile work items: for each system and i-block, its tiles (iblk, jb >= iblk)
-// cut into segments of `seg` tiles; sorted by tile count, largest first
-// (the kernels hand them out dynamically).
 // Spatial order of one system's atoms: recursive bisection of the input
 // positions along the longest side of their bounding box, cut at a multiple
 // of 32 atoms near the middle, so that every 32-atom block is a compact
@@ -343,11 +340,11 @@ static int listed_segment(const std::vector<SysInfo> &sinfo, const std::vector<f
 // Items of the FP64 energy kernels: pairs of i-blocks.  Each item's sums are
 // rounded to fixed point once, so how a system is cut depends on its own size
 // alone and its energies are the same in every batch.  A small system (up to
-// 57 blocks, 870 tiles) waits for its longest item: its tiles' 32 steps are
-// shared by 8, 4 or 2 items in the descreening pass (as many as one resident
-// wave of 1,776 warps holds), and by a thread block's warps in the energy
-// pass (tiles).  A large one takes several tiles per item, which load their i
-// atoms once.
+// 57 blocks, 841 tiles) waits for its longest item: its tiles' 32 steps are
+// shared by 8, 4 or 2 items in the descreening pass (1,680 at 28 and at 40
+// blocks, 1,682 at 57, of the 2,368 warps resident on 148 SMs), and by a
+// thread block's warps in the energy pass (tiles).  A large one takes several
+// tiles per item, which load their i atoms once.
 struct E64Items {
   std::vector<TileItem> born, pair, tiles;
 };
@@ -355,7 +352,7 @@ static E64Items build_items_e64(const std::vector<SysInfo> &sinfo) {
   E64Items out;
   for (int s = 0; s < (int)sinfo.size(); ++s) {
     const int nblk = sinfo[s].nblk;
-    const int parts = nblk <= 28 ? 8 : nblk <= 40 ? 4 : nblk <= 57 ? 2 : 1;  // 224, 440, 870 tiles
+    const int parts = nblk <= 28 ? 8 : nblk <= 40 ? 4 : nblk <= 57 ? 2 : 1;  // 210, 420, 841 tiles
     const int seg = nblk < 160 ? 1 : nblk < 256 ? 2 : nblk < 400 ? 4 : 8;
     const int kn = 32 / parts;
     for (int ib = 0; ib < nblk; ib += 2)
