@@ -1317,7 +1317,7 @@ static int copy_forces(pb2_batch *b, double *forces, cudaStream_t st) {
   return PB2_OK;
 }
 
-// Device-pointer variant: no host copy, no allocation, no synchronisation
+// Device-pointer variant: no host copy, no buffers of its own, no synchronisation
 // (usable from an XLA custom call or under stream capture).
 extern "C" int pb2_energy_forces_device(pb2_batch *b, const double *positions, double *energies,
                                         double *forces, void *stream) {
@@ -1707,7 +1707,7 @@ extern "C" int pb2_min_setup(pb2_batch *b, const uint8_t *heavy, const uint8_t *
   pb2_ctx *ctx = b->ctx;
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   const size_t N = b->n_total;
-  if (!b->m_x0) {
+  if (!b->min_alloc) {
     Dev &D = b->mdev;
     b->m_x0 = D.alloc<double>(3 * N);
     b->m_ft = D.alloc<double>(3 * N);
@@ -1730,13 +1730,15 @@ extern "C" int pb2_min_setup(pb2_batch *b, const uint8_t *heavy, const uint8_t *
     b->m_part = D.alloc<double>(3 * chunks.size());
     b->m_done = D.alloc<int32_t>(b->n_sys);
     b->m_flags = D.alloc<int32_t>(b->n_sys);
-    if (!b->m_chunks || !b->m_chunk0 || !b->m_part || !b->m_done || !b->m_flags)
-      return fail(ctx, PB2_ENOMEM, "minimiser allocation failed");
+    for (const void *p : {(const void *)b->m_x0, (const void *)b->m_ft, (const void *)b->m_xb, (const void *)b->m_best,
+                          (const void *)b->m_par, (const void *)b->m_sys, (const void *)b->m_npos,
+                          (const void *)b->m_sel, (const void *)b->m_chunks, (const void *)b->m_chunk0,
+                          (const void *)b->m_part, (const void *)b->m_done, (const void *)b->m_flags})
+      if (!p) return fail(ctx, PB2_ENOMEM, "minimiser allocation failed");
     int rc;
     if ((rc = upload(ctx, b->m_chunks, chunks)) || (rc = upload(ctx, b->m_chunk0, first))) return rc;
     CUDA_TRY(ctx, cudaMemset(b->m_done, 0, b->n_sys * sizeof(int32_t)));
-    if (!b->m_x0 || !b->m_ft || !b->m_xb || !b->m_best || !b->m_par || !b->m_sys || !b->m_npos || !b->m_sel)
-      return fail(ctx, PB2_ENOMEM, "minimiser allocation failed");
+    b->min_alloc = true;  // a call after one that failed above starts over
   }
   // selections: heavy atoms default to mass > 1.1 amu (prolix simulate.py:596),
   // backbone to the heavy atoms

@@ -158,7 +158,7 @@ struct pb2_batch {
   cudaEvent_t ev_io[3] = {nullptr, nullptr, nullptr};
   // minimiser state (allocated by pb2_min_setup)
   Dev mdev;
-  bool min_ready = false;
+  bool min_ready = false, min_alloc = false;
   double *m_x0 = nullptr, *m_ft = nullptr, *m_xb = nullptr, *m_best = nullptr, *m_par = nullptr;
   double *m_sys = nullptr;  // dt, alpha, best rms, rms, mix_f, mix_p: (6, n_sys)
   int2 *m_chunks = nullptr;
