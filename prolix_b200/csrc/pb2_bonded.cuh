@@ -204,6 +204,13 @@ static __device__ __forceinline__ TermEnergy bonded_term(const BondedArgs &a, in
   }
 }
 
-static __device__ __noinline__ void bonded_term_call(const BondedArgs &a, int t) { bonded_term(a, t); }
+// The out-of-line copy takes the energy where it is wanted, as the bonded
+// kernel does: without it the compiler shares other products of the CMAP
+// polynomial and contracts others into FMAs, and the forces differ from the
+// bonded kernel's in the last bit.
+static __device__ __noinline__ void bonded_term_call(const BondedArgs &a, int t) {
+  const TermEnergy v = bonded_term(a, t);
+  if (v.key >= 0) atomic_add_fix(&a.energy[v.key], v.e);
+}
 
 }  // namespace pb2
