@@ -1261,27 +1261,36 @@ static int enqueue_eval(pb2_batch *b, cudaStream_t st, bool energy) {
   return PB2_OK;
 }
 
-// The same as a graph, for the batches that run by teams: a dozen launches'
-// host time is what a small system's evaluation waits for (166 atoms: 51 us
-// by launches, 37 as a graph; 2,500 atoms, 1,600 tiles: 92 and 100, since
-// consecutive graphs do not overlap).  Captured at the third evaluation (a
-// batch that is evaluated once or twice does not pay for it), as work of this
-// thread alone: a capture in progress on another stream, of this thread or
-// another, neither forbids it nor is ended by it.  NULL: by launches, also
-// where no graph could be made.
+// Adds the launches of `enqueue` to g as a chain of their own.
+template <class F>
+static bool add_chain(cudaGraph_t g, F &&enqueue) {
+  GraphChain c{g};
+  held_chain = &c;
+  const cudaError_t e = enqueue();
+  held_chain = nullptr;
+  return e == cudaSuccess;
+}
+
+// The same as a graph of two chains, for the batches that run by teams: a
+// dozen launches' host time is what a small system's evaluation waits for (166
+// atoms: 51 us by launches, 37 as a graph; 2,500 atoms, 1,600 tiles: 92 and
+// 100, since consecutive graphs do not overlap).  Made at the third evaluation
+// (a batch that is evaluated once or twice does not pay for it), node by node
+// and with the thread's capture mode relaxed: no stream is captured, and a
+// capture in progress elsewhere neither forbids it nor is ended by it.  NULL:
+// by launches, also where no graph could be made.
 static cudaGraphExec_t eval_graph(pb2_batch *b, bool energy) {
   if (!b->team) return nullptr;
   cudaGraphExec_t &ex = b->eval_graphs[energy];
   if (ex || ++b->evals[energy] < 3) return ex;
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
-  cudaStream_t cs = b->cap_stream;
   cudaGraph_t g = nullptr;
-  if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-    const int rc = enqueue_eval(b, cs, energy);
-    if (cudaStreamEndCapture(cs, &g) == cudaSuccess && rc == PB2_OK && cudaGraphInstantiate(&ex, g, 0) != cudaSuccess)
-      ex = nullptr;
-  }
+  if (cudaGraphCreate(&g, 0) != cudaSuccess ||
+      (energy && !add_chain(g, [&] { return enqueue_energy64(b, nullptr); })) ||
+      !add_chain(g, [&] { return enqueue_forces(b, nullptr, energy); }) ||
+      cudaGraphInstantiate(&ex, g, 0) != cudaSuccess)
+    ex = nullptr;
   if (g) cudaGraphDestroy(g);
   cudaThreadExchangeStreamCaptureMode(&mode);
   if (!ex) {

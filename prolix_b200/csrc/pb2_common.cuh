@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <tuple>
+
 #include "prolix_b200.h"
 
 namespace pb2 {
@@ -164,8 +166,48 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // one split, 516 with each kernel's own, 504 at 100 %).
 constexpr unsigned kSmemCarveout = 72;
 
+// A chain of such launches as nodes of a graph instead, while a thread holds a
+// chain: each depends on the one before as it would in a stream.  (Capturing a
+// stream would do the same, but while any stream of the process is being
+// captured, other threads' work on the default stream and waits for the device
+// fail.)
+struct GraphChain {
+  cudaGraph_t graph;
+  cudaGraphNode_t last = nullptr;
+  cudaError_t add(const void *kernel, int grid, int block, void **params) {
+    cudaKernelNodeParams p{};
+    p.func = const_cast<void *>(kernel);
+    p.gridDim = dim3((unsigned)grid);
+    p.blockDim = dim3((unsigned)block);
+    p.kernelParams = params;
+    cudaGraphNode_t node;
+    cudaError_t e = cudaGraphAddKernelNode(&node, graph, nullptr, 0, &p);
+    cudaLaunchAttributeValue v{};
+    v.sharedMemCarveout = kSmemCarveout;
+    if (e == cudaSuccess) e = cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributePreferredSharedMemoryCarveout, &v);
+    if (e == cudaSuccess && last) {
+      cudaGraphEdgeData d{};
+      d.from_port = cudaGraphKernelNodePortProgrammatic;
+      d.type = cudaGraphDependencyTypeProgrammatic;
+      e = cudaGraphAddDependencies_v2(graph, &last, &node, &d, 1);
+    }
+    last = node;
+    return e;
+  }
+};
+inline thread_local GraphChain *held_chain = nullptr;
+
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*kernel)(P...), int grid, int block, cudaStream_t st, const A &...args) {
+  if (held_chain) {
+    std::tuple<P...> values{static_cast<P>(args)...};
+    return std::apply(
+        [&](auto &...v) {
+          void *params[] = {const_cast<void *>(static_cast<const void *>(&v))...};
+          return held_chain->add(reinterpret_cast<const void *>(kernel), grid, block, params);
+        },
+        values);
+  }
   cudaLaunchAttribute at[2] = {};
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
