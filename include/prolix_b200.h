@@ -164,7 +164,7 @@ typedef struct pb2_run_params {
   double skin;          /* A; neighbour-list skin (rebuild when any atom moved > skin/2) */
   int32_t nl_capacity;  /* per-atom neighbour capacity; 0 = automatic */
   int32_t tile_segment; /* tiles per work item; 0 = autotuned/default */
-  int32_t graph_chunk;  /* steps per captured CUDA graph; 0 = 50 */
+  int32_t graph_chunk;  /* steps per CUDA graph; 0 = 50 */
   int32_t partitionable_keys; /* 1: jax_threefry_partitionable layout (JAX default) */
   double gb_cutoff;     /* A; GB pairs and descreening: < 0 same as cutoff, 0 all pairs.
                            prolix's make_energy_fn keeps GB all-pairs while LJ/Coulomb
@@ -300,7 +300,7 @@ int pb2_langevin_run_host(pb2_batch *batch, double *x, double *p, double *f, int
  * at x) are read, n_steps steps run, and the new state is written back into
  * them, all on `stream` without waiting.  This is what a jax.ffi handler
  * binds (XLA owns the buffers).  Steps run as CUDA graphs of up to
- * graph_chunk steps, captured the first time each chunk length is needed:
+ * graph_chunk steps, made the first time each chunk length is needed:
  * make a first call with the same n_steps outside any stream capture. */
 int pb2_langevin_run_device(pb2_batch *batch, double *x, double *p, double *f, int32_t n_steps,
                             void *stream);
@@ -384,7 +384,7 @@ int pb2_get_status(pb2_batch *batch, uint32_t *status, int clear, void *stream);
  * pb2_set_state, pb2_set_full_state or minimisation) opens the next step as
  * it is.  pb2_get_state and pb2_langevin_run_host hand out the uncapped
  * force; a host round trip that passes it back unchanged continues the run
- * exactly.  Setting new limits drops captured graphs.
+ * exactly.  Setting new limits drops the graphs.
  */
 int pb2_set_safeguards(pb2_batch *batch, double vlimit, double max_dx, double force_cap);
 int pb2_get_safeguards(const pb2_batch *batch, double *vlimit, double *max_dx, double *force_cap);
@@ -429,7 +429,7 @@ int pb2_nl_last_build_ms(pb2_batch *batch, double *ms);
  * out[3] chain pass, out[4] bonded, out[5] integrator, out[6] bounding boxes,
  * out[7] whole run. */
 /* Tiles per work item of the pair kernels (the autotuned knob).  Setting it
- * rebuilds the work list and drops captured graphs.  No reference
+ * rebuilds the work list and drops the graphs.  No reference
  * counterpart (prolix's tile sizes are fixed, physics/tiling.py:29-50). */
 int pb2_set_tile_segment(pb2_batch *batch, int32_t segment);
 int pb2_get_tile_segment(const pb2_batch *batch, int32_t *segment);
@@ -464,7 +464,7 @@ int pb2_test_schedule(const pb2_batch *batch, int32_t *pair_list, int32_t *team,
  * blocks per SM its registers are sized for.  Each pass is compiled for a
  * few shapes: pb2_block_shapes fills up to capacity of them and returns how
  * many there are; pb2_set_block_shape picks one (PB2_EINVAL if not
- * compiled) and drops captured graphs.  The autotuner's other knob; no
+ * compiled) and drops the graphs.  The autotuner's other knob; no
  * reference counterpart. */
 int pb2_block_shapes(int32_t pass, int32_t *threads, int32_t *min_blocks, int32_t capacity);
 int pb2_set_block_shape(pb2_batch *batch, int32_t pass, int32_t threads, int32_t min_blocks);
@@ -473,7 +473,7 @@ int pb2_get_block_shape(const pb2_batch *batch, int32_t pass, int32_t *threads, 
 /* I-blocks per warp of the force pass: 2, or 4 (two packed pairs of
  * i-blocks share every j atom's loads; used without a pair list, where the
  * list's rows are pairs of i-blocks).  Both give the same forces and dE/dB
- * bit for bit; setting it drops captured graphs.  No reference
+ * bit for bit; setting it drops the graphs.  No reference
  * counterpart. */
 int pb2_set_force_blocks(pb2_batch *batch, int32_t blocks);
 int pb2_get_force_blocks(const pb2_batch *batch, int32_t *blocks);

@@ -96,7 +96,7 @@ def _time(batch, steps: int) -> float:
   """Mean ms per MD step of ``batch`` as it is configured now."""
   import torch
   stream = torch.cuda.current_stream().cuda_stream
-  batch.langevin_run(1, stream)  # capture
+  batch.langevin_run(1, stream)  # makes the graph
   e0 = torch.cuda.Event(enable_timing=True)
   e1 = torch.cuda.Event(enable_timing=True)
   torch.cuda.synchronize()

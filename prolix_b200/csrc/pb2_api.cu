@@ -1,5 +1,5 @@
 // C ABI of prolix_b200: context and batch management, force evaluation,
-// Langevin runs (captured as CUDA graphs), state access.
+// Langevin runs (replayed as CUDA graphs), state access.
 //
 // Data layout in HBM (batch order = systems concatenated, atoms in input
 // order within a system):
@@ -1075,7 +1075,6 @@ extern "C" int pb2_batch_create(pb2_ctx *ctx, int32_t n_systems, const pb2_syste
   {
     b->fuse = PB2_FUSE_BONDED;  // the autotuner may change this
   }
-  CUDA_TRY(ctx, cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking));
   CUDA_TRY(ctx, cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking));
   for (auto &e : b->ev_side) CUDA_TRY(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   CUDA_TRY(ctx, cudaEventCreate(&b->ev[0]));
@@ -1261,39 +1260,43 @@ static int enqueue_eval(pb2_batch *b, cudaStream_t st, bool energy) {
   return PB2_OK;
 }
 
-// Adds the launches of `enqueue` to g as a chain of their own.
-template <class F>
-static bool add_chain(cudaGraph_t g, F &&enqueue) {
-  GraphChain c{g};
-  held_chain = &c;
-  const cudaError_t e = enqueue();
-  held_chain = nullptr;
-  return e == cudaSuccess;
+// A graph of chains of launches: each of `chains` enqueues one (no stream is
+// captured, see GraphChain).  The thread's capture mode is relaxed meanwhile:
+// a capture in progress elsewhere neither forbids this nor is ended by it.
+template <class... F>
+static cudaError_t build_graph(cudaGraphExec_t *out, F &&...chains) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return e;
+  cudaGraph_t g = nullptr;
+  auto add = [&](auto &&enqueue) {
+    if (e != cudaSuccess) return;
+    GraphChain c{g};
+    held_chain = &c;
+    e = enqueue();
+    held_chain = nullptr;
+  };
+  e = cudaGraphCreate(&g, 0);
+  (add(chains), ...);
+  if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+  if (g) cudaGraphDestroy(g);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) *out = nullptr;
+  return e;
 }
 
 // The same as a graph of two chains, for the batches that run by teams: a
 // dozen launches' host time is what a small system's evaluation waits for (166
 // atoms: 51 us by launches, 37 as a graph; 2,500 atoms, 1,600 tiles: 92 and
 // 100, since consecutive graphs do not overlap).  Made at the third evaluation
-// (a batch that is evaluated once or twice does not pay for it), node by node
-// and with the thread's capture mode relaxed: no stream is captured, and a
-// capture in progress elsewhere neither forbids it nor is ended by it.  NULL:
-// by launches, also where no graph could be made.
+// (a batch that is evaluated once or twice does not pay for it).  NULL: by
+// launches, also where no graph could be made.
 static cudaGraphExec_t eval_graph(pb2_batch *b, bool energy) {
   if (!b->team) return nullptr;
   cudaGraphExec_t &ex = b->eval_graphs[energy];
   if (ex || ++b->evals[energy] < 3) return ex;
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
-  cudaGraph_t g = nullptr;
-  if (cudaGraphCreate(&g, 0) != cudaSuccess ||
-      (energy && !add_chain(g, [&] { return enqueue_energy64(b, nullptr); })) ||
-      !add_chain(g, [&] { return enqueue_forces(b, nullptr, energy); }) ||
-      cudaGraphInstantiate(&ex, g, 0) != cudaSuccess)
-    ex = nullptr;
-  if (g) cudaGraphDestroy(g);
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  if (!ex) {
+  const auto energies = [&] { return energy ? enqueue_energy64(b, nullptr) : cudaSuccess; };
+  if (build_graph(&ex, energies, [&] { return enqueue_forces(b, nullptr, energy); }) != cudaSuccess) {
     cudaGetLastError();   // the launches report their own
     b->evals[energy] = 0;  // and the third call from here tries again
   }
@@ -1434,27 +1437,18 @@ static int get_graph(pb2_batch *b, int chunk, int parity, cudaGraphExec_t *out) 
     *out = it->second;
     return PB2_OK;
   }
-  cudaStream_t cs = b->cap_stream;
-  CUDA_TRY(ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-  cudaError_t err = cudaSuccess;
-  int p = parity;
-  for (int t = 0; t < chunk && err == cudaSuccess; ++t) {
-    err = launch_step(int_args(b, p, t > 0), cs);
-    if (err == cudaSuccess) err = enqueue_forces(b, cs, false);
-    p ^= 1;
-  }
-  if (err == cudaSuccess) err = launch_finish(int_args(b, p, 0), cs);
-  cudaGraph_t g = nullptr;
-  cudaError_t e2 = cudaStreamEndCapture(cs, &g);
-  if (err != cudaSuccess || e2 != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
-    return fail(ctx, PB2_ECUDA, std::string("graph capture failed: ") +
-                                    cudaGetErrorString(err != cudaSuccess ? err : e2));
-  }
   cudaGraphExec_t ex = nullptr;
-  cudaError_t e3 = cudaGraphInstantiate(&ex, g, 0);
-  cudaGraphDestroy(g);
-  if (e3 != cudaSuccess) return fail(ctx, PB2_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e3));
+  const cudaError_t e = build_graph(&ex, [&] {
+    cudaError_t err = cudaSuccess;
+    int p = parity;
+    for (int t = 0; t < chunk && err == cudaSuccess; ++t) {
+      err = launch_step(int_args(b, p, t > 0), nullptr);
+      if (err == cudaSuccess) err = enqueue_forces(b, nullptr, false);
+      p ^= 1;
+    }
+    return err == cudaSuccess ? launch_finish(int_args(b, p, 0), nullptr) : err;
+  });
+  if (e != cudaSuccess) return fail(ctx, PB2_ECUDA, std::string("step graph: ") + cudaGetErrorString(e));
   b->graphs[key] = ex;
   *out = ex;
   return PB2_OK;
@@ -1778,30 +1772,17 @@ static int min_graph(pb2_batch *b, int mode, int chunk, cudaGraphExec_t *out) {
     return PB2_OK;
   }
   const MinArgs ma = min_args(b);
-  cudaStream_t cs = b->cap_stream;
-  CUDA_TRY(ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
-  cudaError_t err = cudaSuccess;
-  for (int t = 0; t < chunk && err == cudaSuccess; ++t) {
-    if (mode == 0) {
-      err = launch_min(kMinOpSd, ma, nullptr, cs);
-      if (err == cudaSuccess) err = enqueue_forces(b, cs, false);
-    } else {
-      err = launch_min(kMinOpFireMove, ma, nullptr, cs);
-      if (err == cudaSuccess) err = enqueue_forces(b, cs, false);
-      if (err == cudaSuccess) err = launch_min(kMinOpFireClose, ma, nullptr, cs);
-    }
-  }
-  cudaGraph_t g = nullptr;
-  cudaError_t e2 = cudaStreamEndCapture(cs, &g);
-  if (err != cudaSuccess || e2 != cudaSuccess) {
-    if (g) cudaGraphDestroy(g);
-    return fail(ctx, PB2_ECUDA, std::string("graph capture failed: ") +
-                                    cudaGetErrorString(err != cudaSuccess ? err : e2));
-  }
   cudaGraphExec_t ex = nullptr;
-  cudaError_t e3 = cudaGraphInstantiate(&ex, g, 0);
-  cudaGraphDestroy(g);
-  if (e3 != cudaSuccess) return fail(ctx, PB2_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e3));
+  const cudaError_t e = build_graph(&ex, [&] {
+    cudaError_t err = cudaSuccess;
+    for (int t = 0; t < chunk && err == cudaSuccess; ++t) {
+      err = launch_min(mode == 0 ? kMinOpSd : kMinOpFireMove, ma, nullptr, nullptr);
+      if (err == cudaSuccess) err = enqueue_forces(b, nullptr, false);
+      if (err == cudaSuccess && mode != 0) err = launch_min(kMinOpFireClose, ma, nullptr, nullptr);
+    }
+    return err;
+  });
+  if (e != cudaSuccess) return fail(ctx, PB2_ECUDA, std::string("minimiser graph: ") + cudaGetErrorString(e));
   b->min_graphs[key] = ex;
   *out = ex;
   return PB2_OK;
@@ -2093,7 +2074,7 @@ extern "C" int pb2_set_safeguards(pb2_batch *b, double vlimit, double max_dx, do
   CUDA_TRY(ctx, cudaSetDevice(ctx->device));
   CUDA_TRY(ctx, cudaDeviceSynchronize());
   for (int k = 0; k < 3; ++k) b->guard[k] = g[k];
-  for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);  // they captured the old limits
+  for (auto &kv : b->graphs) cudaGraphExecDestroy(kv.second);  // they hold the old limits
   b->graphs.clear();
   return PB2_OK;
 }
@@ -2136,7 +2117,7 @@ extern "C" int pb2_set_tile_segment(pb2_batch *b, int32_t segment) {
   b->params.tile_segment = segment;
   if (int rc = setup_items2(b, segment)) return rc;
   if (int rc = setup_pair_list(b, segment)) return rc;
-  b->drop_graphs();  // they captured the old list
+  b->drop_graphs();  // they hold the old list
   return PB2_OK;
 }
 
@@ -2216,7 +2197,7 @@ extern "C" int pb2_set_block_shape(pb2_batch *b, int32_t pass, int32_t threads, 
     b->shape[pass] = found;
     set_pair_grid(b, pass);
   }
-  b->drop_graphs();  // they captured the old kernel
+  b->drop_graphs();  // they hold the old kernel
   return PB2_OK;
 }
 
@@ -2235,7 +2216,7 @@ extern "C" int pb2_set_force_blocks(pb2_batch *b, int32_t blocks) {
   CUDA_TRY(b->ctx, cudaSetDevice(b->ctx->device));
   CUDA_TRY(b->ctx, cudaDeviceSynchronize());
   b->force_blocks = blocks;
-  b->drop_graphs();  // they captured the other kernel
+  b->drop_graphs();  // they hold the other kernel
   return PB2_OK;
 }
 
@@ -2251,7 +2232,7 @@ extern "C" int pb2_set_fusion(pb2_batch *b, int32_t flags) {
   CUDA_TRY(b->ctx, cudaSetDevice(b->ctx->device));
   CUDA_TRY(b->ctx, cudaDeviceSynchronize());
   b->fuse = flags;
-  b->drop_graphs();  // they captured the old schedule
+  b->drop_graphs();  // they hold the old schedule
   return PB2_OK;
 }
 

@@ -142,7 +142,6 @@ struct pb2_batch {
   int grid_bonded = 1;
   int team = 0;                  // warps per tile of the pair passes (0: one, tile2_kernel)
   int grid_team[3] = {1, 1, 1};
-  cudaStream_t cap_stream = nullptr;
   std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
   // evaluations without and with energies: graph, and calls before it
   cudaGraphExec_t eval_graphs[2] = {nullptr, nullptr};
@@ -198,7 +197,7 @@ struct pb2_batch {
   cudaEvent_t nl_ev[2] = {nullptr, nullptr};  // around the last build's launches
   bool nl_timed = false;
 
-  // Every captured graph (their kernels, shapes and work lists are fixed).
+  // Every graph (their kernels, shapes and work lists are fixed).
   void drop_graphs() {
     for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
     graphs.clear();
@@ -212,7 +211,6 @@ struct pb2_batch {
 
   ~pb2_batch() {
     drop_graphs();
-    if (cap_stream) cudaStreamDestroy(cap_stream);
     if (side) cudaStreamDestroy(side);
     for (auto &e : ev_side)
       if (e) cudaEventDestroy(e);

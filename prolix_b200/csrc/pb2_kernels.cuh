@@ -203,7 +203,7 @@ struct IntArgs {
 // warn_counts columns (prolix typing.py:559-563) and their warn_flags bits
 enum { kWarnVlimit = 0, kWarnForceCap = 1, kWarnConstr = 2, kWarnDxCap = 3, kWarnTypes = 4 };
 // Minimiser (pb2_minimize.cu).  Stage parameters live in device memory
-// (par[kMin*]) so that captured graphs serve every stage.
+// (par[kMin*]) so that one graph serves every stage.
 enum { kMinK = 0, kMinKind, kMinSdDt, kMinMaxDx, kMinDtStart, kMinDtMax, kMinMaxDisp, kMinForceCap, kMinNPar };
 enum { kMinOpSd = 0, kMinOpRollback, kMinOpFireInit, kMinOpFireMove, kMinOpFireClose, kMinOpFireEnd,
        kMinOpTakeBest, kMinOpRms };

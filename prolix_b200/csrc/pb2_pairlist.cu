@@ -18,9 +18,9 @@
 // minimiser's, or place_kernel at the start of an evaluation) raises the
 // rebuild flag when one is more than skin/2 from its position at the last
 // build, and this kernel, launched every step of a run with a list (inside
-// the captured graphs), returns at once unless the flag is set.  A rebuild writes the new items into the buffer the pair kernels
-// are not reading, and the last warp to finish publishes it, so no launch
-// needs the host.
+// the graphs), returns at once unless the flag is set.  A rebuild writes the
+// new items into the buffer the pair kernels are not reading, and the last
+// warp to finish publishes it, so no launch needs the host.
 #include "pb2_common.cuh"
 #include "pb2_kernels.cuh"
 

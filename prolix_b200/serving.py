@@ -15,7 +15,7 @@ a cohort whose requests have all ended is released.
 
 The step count of a tick is the largest of chunk, chunk/2, chunk/5,
 chunk/10, 1 (and 1-step divisions thereof) that does not pass the nearest
-completion, so every cohort captures at most a handful of step graphs.
+completion, so every cohort makes at most a handful of step graphs.
 
 Systems never interact and forces use order-independent fixed-point sums,
 so a request's result is bit-identical whether it ran alone or in any mix
